@@ -68,14 +68,14 @@ u64 host_fmix64(u64 x) {
     return x;
 }
 
-// The level kernel's exact-key fingerprint of a CS (n words, zero padding up to pitch): word i
-// adds (lo(w) + lo(k)) * (hi(w) + hi(k)) with k = (i + 1) * 0x9E3779B97F4A7C15 (32-bit sums,
+// The level kernel's exact-key fingerprint of a CS (n words, zero padding up to pitch), taken
+// on row words (reversed positions): word i adds (lo(w) + lo(k)) * (hi(w) + hi(k)) with k = (i + 1) * 0x9E3779B97F4A7C15 (32-bit sums,
 // 64-bit product), and the sum goes through fmix64.  The device adds the same terms in
 // another order; the sum is the same modulo 2^64.
 u64 host_fingerprint_exact(const uint64_t *w, int n, int pitch) {
     u64 sum = 0;
     for (int i = 0; i < pitch; ++i) {
-        const u64 v = i < n ? w[i] : 0ull, k = (u64)(i + 1) * 0x9E3779B97F4A7C15ull;
+        const u64 v = i < n ? reverse_positions(w[i]) : 0ull, k = (u64)(i + 1) * 0x9E3779B97F4A7C15ull;
         sum += (u64)((u32)v + (u32)k) * (u64)((u32)(v >> 32) + (u32)(k >> 32));
     }
     return host_fmix64(sum);
@@ -456,9 +456,9 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
         for (int i = 0; i < n; ++i) {
             u64 w = 0;
             for (int k = t->offsets[i]; k < t->offsets[i + 1]; ++k)
-                if (t->steps[k] & bit) w |= 1ull << (k - t->offsets[i]);
+                if (t->steps[k] & bit) w |= 1ull << (62 - (k - t->offsets[i]));
             letters[(size_t)j * pitch + i] = w;
-            if (i < npos ? !(w & 1) : (w & 1)) acc = false;
+            if (((w >> 62) != 0) != (i < npos)) acc = false;
         }
         all++;
         if (acc && letter_hit < 0) {
@@ -516,7 +516,7 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
     std::vector<u32> kmeta(pitch, 0u);
     for (int i = 0; i < n; ++i) {
         const int ln = t->offsets[i + 1] - t->offsets[i];
-        wmeta[i] = (ln >= 63 ? 0x7FFFFFFFFFFFFFFFull : ((1ull << ln) - 1)) | (i < npos ? (1ull << 63) : 0ull);
+        wmeta[i] = row_lenmask(ln) | (i < npos ? (1ull << 63) : 0ull);
     }
     int rlx_type = 0;
     if (ref_keys) {
@@ -1426,7 +1426,8 @@ LTLG_API int ltlg_engine_read_rows(ltlg_engine *e, int64_t first, int64_t count,
                          cudaMemcpyDeviceToHost);
         if (err != cudaSuccess) return fail_cuda(e, err, nullptr);
         for (int64_t r = 0; r < count; ++r)
-            memcpy(rows + (size_t)r * e->n, tmp.data() + (size_t)r * e->pitch, (size_t)e->n * 8);
+            for (int i = 0; i < e->n; ++i)
+                rows[(size_t)r * e->n + i] = reverse_positions(tmp[(size_t)r * e->pitch + i]);
     }
     if (parents) {
         err = cudaMemcpy(parents, (u64 *)e->parents.p + first, (size_t)count * 8, cudaMemcpyDeviceToHost);

@@ -100,9 +100,9 @@ struct BinGen {
     __device__ __forceinline__ ulonglong2 word(int t, int c, ulonglong2 r) const {
         if (OPC == OP_U) {
             const ulonglong2 l = left[(t >> 1) * nch + c];
-            const u64 lx = rev62(l.x), ly = rev62(l.y), rx = rev62(r.x), ry = rev62(r.y);
-            if (t & 1) return make_ulonglong2(until_rev(lx | rx, lx), until_rev(ly | ry, ly));
-            return make_ulonglong2(until_rev(lx | rx, rx), until_rev(ly | ry, ry));
+            const u64 ax = l.x | r.x, ay = l.y | r.y;
+            if (t & 1) return make_ulonglong2(row_until(ax, l.x), row_until(ay, l.y));
+            return make_ulonglong2(row_until(ax, r.x), row_until(ay, r.y));
         }
         const ulonglong2 l = left[t * nch + c];
         return rop == OP_AND ? make_ulonglong2(l.x & r.x, l.y & r.y) : make_ulonglong2(l.x | r.x, l.y | r.y);
@@ -120,7 +120,7 @@ struct UnGen {
     __device__ __forceinline__ Pre pre(int c) const { return UnPre{__ldcg(meta + c), __ldcg(src + c)}; }
     __device__ __forceinline__ ulonglong2 word(int t, int, const Pre &p) const {
         const int op = unary_slot_op(t);
-        return make_ulonglong2(unary_word(op, p.s.x, p.m.x & LENMASK), unary_word(op, p.s.y, p.m.y & LENMASK));
+        return make_ulonglong2(row_unary(op, p.s.x, p.m.x & LENMASK), row_unary(op, p.s.y, p.m.y & LENMASK));
     }
 };
 
@@ -143,7 +143,7 @@ __device__ void ref_key(const InstArgs &A, const Gen &g, int t, int lane, u64 &k
         for (int e = 0; e < 2; ++e) {
             const int i = 2 * c + e;
             if (i >= A.n) break;
-            const u64 w = e ? w2.y : w2.x;
+            const u64 w = rev62(e ? w2.y : w2.x);  // the reference's bit order
             if (A.rlx_type == 3) {
                 // splitmix64 finaliser per word, folded by halves (ltli6463.cu:108-119)
                 u64 x = w;
@@ -410,13 +410,22 @@ __device__ __forceinline__ void resolve(const InstArgs &A, InstCtl *C, int cost,
 }
 
 // Fingerprints, acceptance, the find record, uniqueness for NC candidates of one warp.
-// pos_of(t): block position of candidate t (the find record is per block).
+// fails[t]: this lane's words of candidate t at position 0 (fails2); bp, bn: the row statistics'
+// bits (pmiss2, nhit2), kept only when the learn counts them.  pos_of(t): block position of candidate t (the find record is per block).
 template <int NC, class Gen, class ParentOf, class PosOf, class TidOf>
-__device__ __forceinline__ void finish(const InstArgs &A, InstCtl *C, Slot &sl, const Gen &g, u64 (&h)[NC], u32 bp,
-                                       u32 bn, u32 valid, ParentOf parent_of, PosOf pos_of, TidOf tid_of, int lane) {
+__device__ __forceinline__ void finish(const InstArgs &A, InstCtl *C, Slot &sl, const Gen &g, u64 (&h)[NC],
+                                       u32 (&fails)[NC], u32 bp, u32 bn, u32 valid, ParentOf parent_of, PosOf pos_of,
+                                       TidOf tid_of, int lane) {
     const u64 sum = reduce_to_lane<NC>(h, lane);
-    const u32 anyp = __reduce_or_sync(FULL, bp), anyn = __reduce_or_sync(FULL, bn);
-    const u32 acc = ~(anyp | anyn) & valid;
+    u32 fb = 0;
+#pragma unroll
+    for (int t = 0; t < NC; ++t) fb |= (fails[t] & ROW_BIT0_HI) ? 1u << t : 0u;
+    const u32 acc = ~__reduce_or_sync(FULL, fb) & valid;
+    u32 anyp = 0, anyn = 0;
+    if (A.lstats) {
+        anyp = __reduce_or_sync(FULL, bp);
+        anyn = __reduce_or_sync(FULL, bn);
+    }
     const u64 myparent = parent_of(lane);
     const int cost = sl.cost;
     if (acc) {
@@ -469,8 +478,13 @@ __device__ __forceinline__ void binary_row(const InstArgs &A, InstCtl *C, Slot &
     const int nch = A.pitch >> 1, npos = A.npos, n = A.n;
     const int rop = sl.op;
     u64 h[NC];
+    u32 fails[NC];
 #pragma unroll
-    for (int t = 0; t < NC; ++t) h[t] = 0;
+    for (int t = 0; t < NC; ++t) {
+        h[t] = 0;
+        fails[t] = 0;
+    }
+    const bool stats = A.lstats != nullptr;
     u32 bp = 0, bn = 0;
     constexpr int CH = 2;  // right-row chunks in flight per lane
     for (int c0 = lane; c0 < nch; c0 += 32 * CH) {
@@ -486,28 +500,28 @@ __device__ __forceinline__ void binary_row(const InstArgs &A, InstCtl *C, Slot &
             if (c >= nch) continue;
             const u64 k = (2ull * (u64)c + 1ull) * WEYL;
             const ulonglong2 rv = rvv[u];
-            const u64 p0 = 2 * c < npos ? 1ull : 0ull, p1 = 2 * c + 1 < npos ? 1ull : 0ull;
+            const u32 p0 = 2 * c < npos ? ROW_BIT0_HI : 0u, p1 = 2 * c + 1 < npos ? ROW_BIT0_HI : 0u;
             const bool v0 = 2 * c < n, v1 = 2 * c + 1 < n;
-            const u64 rx = OPC == OP_U ? rev62(rv.x) : 0ull, ry = OPC == OP_U ? rev62(rv.y) : 0ull;
+            auto take = [&](int t, u64 w0, u64 w1) {
+                h[t] += hw<HK>(w0, k, v0) + hw<HK>(w1, k + WEYL, v1);
+                fails[t] |= fails2(w0, w1, p0, p1);
+                if (stats) {
+                    bp |= pmiss2(w0, w1, p0, p1) << t;
+                    bn |= nhit2(w0, w1, p0, p1) << t;
+                }
+            };
 #pragma unroll
             for (int t = 0; t < TLP; ++t) {
                 if (t < nl) {
                     const ulonglong2 lv = tile[t * nch + c];
                     if (OPC == OP_U) {
-                        const u64 lx = rev62(lv.x), ly = rev62(lv.y);
-                        const u64 ax = lx | rx, ay = ly | ry;
-                        const u64 a0 = until_rev(ax, rx), a1 = until_rev(ay, ry);  // l U r
-                        const u64 b0 = until_rev(ax, lx), b1 = until_rev(ay, ly);  // r U l
-                        h[2 * t] += hw<HK>(a0, k, v0) + hw<HK>(a1, k + WEYL, v1);
-                        h[2 * t + 1] += hw<HK>(b0, k, v0) + hw<HK>(b1, k + WEYL, v1);
-                        bp |= (pmiss2(a0, a1, p0, p1) << (2 * t)) | (pmiss2(b0, b1, p0, p1) << (2 * t + 1));
-                        bn |= (nhit2(a0, a1, p0, p1) << (2 * t)) | (nhit2(b0, b1, p0, p1) << (2 * t + 1));
+                        const u64 ax = lv.x | rv.x, ay = lv.y | rv.y;
+                        take(2 * t, row_until(ax, rv.x), row_until(ay, rv.y));      // l U r
+                        take(2 * t + 1, row_until(ax, lv.x), row_until(ay, lv.y));  // r U l
+                    } else if (rop == OP_AND) {
+                        take(t, lv.x & rv.x, lv.y & rv.y);
                     } else {
-                        const u64 w0 = rop == OP_AND ? (lv.x & rv.x) : (lv.x | rv.x);
-                        const u64 w1 = rop == OP_AND ? (lv.y & rv.y) : (lv.y | rv.y);
-                        h[t] += hw<HK>(w0, k, v0) + hw<HK>(w1, k + WEYL, v1);
-                        bp |= pmiss2(w0, w1, p0, p1) << t;
-                        bn |= nhit2(w0, w1, p0, p1) << t;
+                        take(t, lv.x | rv.x, lv.y | rv.y);
                     }
                 }
             }
@@ -516,7 +530,7 @@ __device__ __forceinline__ void binary_row(const InstArgs &A, InstCtl *C, Slot &
     const int cnt = OPC == OP_U ? 2 * nl : nl;
     const u32 valid = cnt >= 32 ? FULL : ((1u << cnt) - 1u);
     const BinGen<OPC> g{tile, R, nch, rop};
-    finish<NC>(A, C, sl, g, h, bp, bn, valid,
+    finish<NC>(A, C, sl, g, h, fails, bp, bn, valid,
                [&](int t) {
                    if (OPC == OP_U) {
                        const u64 l = (u64)(l_first + (t >> 1));
@@ -542,6 +556,8 @@ __device__ __forceinline__ void unary_row(const InstArgs &A, InstCtl *C, Slot &s
     const int nch = A.pitch >> 1, npos = A.npos, n = A.n;
     const ulonglong2 *meta = reinterpret_cast<const ulonglong2 *>(A.wmeta);
     u64 h[NC] = {0, 0, 0, 0};
+    u32 fails[NC] = {0, 0, 0, 0};
+    const bool stats = A.lstats != nullptr;
     u32 bp = 0, bn = 0;
     constexpr int CH = 2;  // source-row chunks in flight per lane
     for (int c0 = lane; c0 < nch; c0 += 32 * CH) {
@@ -559,24 +575,27 @@ __device__ __forceinline__ void unary_row(const InstArgs &A, InstCtl *C, Slot &s
             const int c = c0 + 32 * u;
             if (c >= nch) continue;
             const u64 k = (2ull * (u64)c + 1ull) * WEYL;
-            const u64 p0 = 2 * c < npos ? 1ull : 0ull, p1 = 2 * c + 1 < npos ? 1ull : 0ull;
+            const u32 p0 = 2 * c < npos ? ROW_BIT0_HI : 0u, p1 = 2 * c + 1 < npos ? ROW_BIT0_HI : 0u;
             const bool v0 = 2 * c < n, v1 = 2 * c + 1 < n;
             const u64 m0 = mv[u].x & LENMASK, m1 = mv[u].y & LENMASK;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 if ((mask >> j) & 1) {
                     const int op = unary_slot_op(j);
-                    const u64 w0 = unary_word(op, sv[u].x, m0), w1 = unary_word(op, sv[u].y, m1);
+                    const u64 w0 = row_unary(op, sv[u].x, m0), w1 = row_unary(op, sv[u].y, m1);
                     h[j] += hw<HK>(w0, k, v0) + hw<HK>(w1, k + WEYL, v1);
-                    bp |= pmiss2(w0, w1, p0, p1) << j;
-                    bn |= nhit2(w0, w1, p0, p1) << j;
+                    fails[j] |= fails2(w0, w1, p0, p1);
+                    if (stats) {
+                        bp |= pmiss2(w0, w1, p0, p1) << j;
+                        bn |= nhit2(w0, w1, p0, p1) << j;
+                    }
                 }
             }
         }
     }
     const u32 valid = (u32)(mask & 15);
     const UnGen g{src, meta};
-    finish<NC>(A, C, sl, g, h, bp, bn, valid,
+    finish<NC>(A, C, sl, g, h, fails, bp, bn, valid,
                [&](int t) { return pack_parent(unary_slot_op(t & 3), (u64)s, 0); },
                [&](int t) { return sl.upos[t & 3]; }, [&](int) -> u64 { return (u64)(s - sl.e_r0); }, lane);
     if (lane == 0) atomicAdd(&sl.evals, (unsigned)__popc(valid));
@@ -1092,8 +1111,8 @@ __device__ bool setup_instance(BatchDev &B, int s, int idx, int lane) {
             if (i < n) {
                 const int a = offs[i], b = offs[i + 1];
                 for (int k = a; k < b; ++k)
-                    if (steps[k] & bit) w |= 1ull << (k - a);
-                if (i < npos ? !(w & 1ull) : (w & 1ull)) acc = false;
+                    if (steps[k] & bit) w |= 1ull << (62 - (k - a));
+                if (((w >> 62) != 0) != (i < npos)) acc = false;
             }
             __stcg(A.cache + (u64)j * pitch + i, w);
         }
@@ -1124,7 +1143,7 @@ __device__ bool setup_instance(BatchDev &B, int s, int idx, int lane) {
         u64 m = 0;
         if (i < n) {
             const int ln = offs[i + 1] - offs[i];
-            m = (ln >= 63 ? 0x7FFFFFFFFFFFFFFFull : ((1ull << ln) - 1)) | (i < npos ? (1ull << 63) : 0ull);
+            m = row_lenmask(ln) | (i < npos ? (1ull << 63) : 0ull);
         }
         __stcg(const_cast<u64 *>(A.wmeta) + i, m);
     }
@@ -1721,7 +1740,7 @@ __global__ void insert_letters_kernel(const InstArgs *__restrict__ pA, int nalph
             const u64 k = (2ull * (u64)c + 1ull) * WEYL;
             const ulonglong2 w = reinterpret_cast<const ulonglong2 *>(row)[c];
             h[0] += hw<HK>(w.x, k, 2 * c < A.n) + hw<HK>(w.y, k + WEYL, 2 * c + 1 < A.n);
-            const u64 p0 = 2 * c < A.npos ? 1ull : 0ull, p1 = 2 * c + 1 < A.npos ? 1ull : 0ull;
+            const u32 p0 = 2 * c < A.npos ? ROW_BIT0_HI : 0u, p1 = 2 * c + 1 < A.npos ? ROW_BIT0_HI : 0u;
             pm |= pmiss2(w.x, w.y, p0, p1);
             nh |= nhit2(w.x, w.y, p0, p1);
         }
@@ -1843,7 +1862,7 @@ __global__ void apply_op_kernel(int op, const u64 *a, const u64 *b, const u64 *w
         case OP_NEG:
         case OP_X:
         case OP_F:
-        case OP_G: w = unary_word(op, x, m); break;
+        case OP_G: w = unary_bits(op, x, m); break;
         case OP_AND: w = x & y; break;
         case OP_OR: w = x | y; break;
         case OP_U:
@@ -1886,7 +1905,7 @@ __global__ void eval_formula_kernel(const int *__restrict__ prog, int len, const
         if (op == OP_ATOM) {
             v = atoms[(u64)arg * n + t];
         } else if (op == OP_NEG || op == OP_X || op == OP_F || op == OP_G) {
-            v = unary_word(op, stack[(u64)(sp - 1) * n + t], m);
+            v = unary_bits(op, stack[(u64)(sp - 1) * n + t], m);
             --sp;
         } else {
             const u64 y = stack[(u64)(sp - 1) * n + t], x = stack[(u64)(sp - 2) * n + t];

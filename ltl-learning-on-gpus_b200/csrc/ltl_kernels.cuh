@@ -45,6 +45,18 @@ __host__ __device__ inline u64 parent_right(u64 p) { return p & 0x3FFFFFFFull; }
 // Operator of slot j of a fused unary entry: 0 ~, 1 X, 2 F, 3 G.
 __host__ __device__ inline int unary_slot_op(int j) { return j == 0 ? OP_NEG : j == 1 ? OP_X : j == 2 ? OP_F : OP_G; }
 
+// Length mask of a trace of ln steps in row words (position k is bit 62 - k).
+__host__ __device__ inline u64 row_lenmask(int ln) {
+    return ln >= 63 ? 0x7FFFFFFFFFFFFFFFull : 0x7FFFFFFFFFFFFFFFull & ~((1ull << (63 - ln)) - 1ull);
+}
+// A CS word in the other bit order (positions 0 .. 62; its own inverse).
+inline u64 reverse_positions(u64 w) {
+    w = ((w >> 1) & 0x5555555555555555ull) | ((w & 0x5555555555555555ull) << 1);
+    w = ((w >> 2) & 0x3333333333333333ull) | ((w & 0x3333333333333333ull) << 2);
+    w = ((w >> 4) & 0x0F0F0F0F0F0F0F0Full) | ((w & 0x0F0F0F0F0F0F0F0Full) << 4);
+    return __builtin_bswap64(w) >> 1;
+}
+
 constexpr int POS_NONE = 0x7FFFFFFF;
 constexpr int LSTATS = 2;              // row-statistics counters per cost (see count_row_stats)
 constexpr u64 NO_FIND = ~0ull;         // InstCtl::found_key before any find

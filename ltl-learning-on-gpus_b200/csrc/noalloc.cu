@@ -157,9 +157,9 @@ extern "C" LTLG_API int ltlg_learn_noalloc(const ltlg_traces *t, const ltlg_opti
         for (int i = 0; i < n; ++i) {
             u64 w = 0;
             for (int k = t->offsets[i]; k < t->offsets[i + 1]; ++k)
-                if (t->steps[k] & bit) w |= 1ull << (k - t->offsets[i]);
+                if (t->steps[k] & bit) w |= 1ull << (62 - (k - t->offsets[i]));
             letters[j * pitch + i] = w;
-            if (i < npos ? !(w & 1) : (w & 1)) acc = false;
+            if (((w >> 62) != 0) != (i < npos)) acc = false;
         }
         ++all;
         if (acc && letter_hit < 0) {
@@ -243,7 +243,7 @@ extern "C" LTLG_API int ltlg_learn_noalloc(const ltlg_traces *t, const ltlg_opti
     memset(wm, 0, sizeof(wm));
     for (int i = 0; i < n; ++i) {
         const int ln = t->offsets[i + 1] - t->offsets[i];
-        wm[i] = (ln >= 63 ? 0x7FFFFFFFFFFFFFFFull : ((1ull << ln) - 1)) | (i < npos ? (1ull << 63) : 0ull);
+        wm[i] = row_lenmask(ln) | (i < npos ? (1ull << 63) : 0ull);
     }
     InstCtl hc;
     memset(&hc, 0, sizeof(hc));

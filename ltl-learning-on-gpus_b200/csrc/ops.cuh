@@ -44,20 +44,42 @@ __device__ __forceinline__ u64 glob_bits(u64 w, u64 m) {
 // bits 62..0 (bit 63 of every CS is 0) so the carry into bit 63 holds position 0.  Same
 // result as the doubling recurrence of ltli6463.cu:739-752.
 __device__ __forceinline__ u64 rev62(u64 v) { return __brevll(v) >> 1; }
-__device__ __forceinline__ u64 until_rev(u64 a, u64 yr) {  // a = xr | yr
-    return __brevll(((a + yr) ^ a ^ yr) & ~1ull);
-}
 __device__ __forceinline__ u64 until_bits(u64 x, u64 y) {
-    const u64 xr = rev62(x), yr = rev62(y);
-    return until_rev(xr | yr, yr);
+    const u64 xr = rev62(x), yr = rev62(y), a = xr | yr;
+    return __brevll(((a + yr) ^ a ^ yr) & ~1ull);
 }
 
 // Unary operator op (OP_NEG, OP_X, OP_F, OP_G) on one word with its length mask m.
-__device__ __forceinline__ u64 unary_word(int op, u64 w, u64 m) {
+__device__ __forceinline__ u64 unary_bits(int op, u64 w, u64 m) {
     if (op == OP_NEG) return ~w & m;
     if (op == OP_X) return w >> 1;
     if (op == OP_F) return fin_bits(w);
     return glob_bits(w, m);
+}
+
+// ---- Row words.  The language cache holds every word bit-reversed (rev62): position k of a
+// trace is bit 62 - k, so later positions are lower bits.  U is then one addition, F and G are
+// the two's-complement lowest-set-bit forms, and no operator needs a bit reversal or a leading-
+// zero count, which run at a quarter of the rate of adds and logic on sm_100a.  Length masks
+// (InstArgs::wmeta) are reversed the same way; rows are reversed back where they leave the
+// library (ltlg_engine_read_rows) and for the reference's relaxed keys (ref_key).
+// Measured on whole learns against rows in natural order: 1000 traces to cost 8 (243 thousand
+// candidates) 1.43 -> 1.35 ms, 4000 traces (602 thousand) 10.74 -> 10.45 ms.
+constexpr u32 ROW_BIT0_HI = 0x40000000u;  // position 0 in a row word's upper half
+
+__device__ __forceinline__ u64 row_until(u64 a, u64 y) {  // x U y, a = x | y
+    return ((a + y) ^ a ^ y) >> 1;
+}
+// F: every position at or before the last one where the operand holds: the bits at and above
+// the lowest set bit.  G: the positions after the last one (inside the trace) where it fails:
+// the operand's bits below the lowest set bit of z = ~w & m, all of them when z is 0 (the bits of
+// z - 1 above that one are z's, which are not the operand's).
+__device__ __forceinline__ u64 row_unary(int op, u64 w, u64 m) {
+    if (op == OP_NEG) return ~w & m;
+    if (op == OP_X) return (w << 1) & M63;
+    if (op == OP_F) return (w | (0ull - w)) & M63;
+    const u64 z = ~w & m;
+    return w & (z - 1ull);
 }
 
 // Word i (key = (i + 1) * WEYL) of a CS adds to the fingerprint sum:
@@ -70,13 +92,16 @@ __device__ __forceinline__ u64 hw(u64 w, u64 key, bool valid) {
     return valid ? fmix64(w ^ key) : 0ull;
 }
 
-// Acceptance at position 0 for a pair of words whose traces are positive (p = 1) or not:
-// a positive trace where the candidate fails, a negative (or padding) trace where it holds.
-__device__ __forceinline__ u32 pmiss2(u64 w0, u64 w1, u64 p0, u64 p1) {
-    return (u32)(((~w0 & p0) | (~w1 & p1)) & 1ull);
+// Acceptance at position 0, kept in bit 30 of the upper halves: p is ROW_BIT0_HI for a positive
+// trace's word and 0 for a negative's (or padding), so a word fails there iff hi(w) ^ p has the
+// bit: a positive where the candidate fails, a negative where it holds.
+__device__ __forceinline__ u32 hi32(u64 w) { return (u32)(w >> 32); }
+__device__ __forceinline__ u32 fails2(u64 w0, u64 w1, u32 p0, u32 p1) { return (hi32(w0) ^ p0) | (hi32(w1) ^ p1); }
+__device__ __forceinline__ u32 pmiss2(u64 w0, u64 w1, u32 p0, u32 p1) {
+    return ((~hi32(w0) & p0) | (~hi32(w1) & p1)) >> 30;
 }
-__device__ __forceinline__ u32 nhit2(u64 w0, u64 w1, u64 p0, u64 p1) {
-    return (u32)(((w0 & ~p0) | (w1 & ~p1)) & 1ull);
+__device__ __forceinline__ u32 nhit2(u64 w0, u64 w1, u32 p0, u32 p1) {
+    return (((hi32(w0) & ~p0) | (hi32(w1) & ~p1)) >> 30) & 1u;
 }
 
 __device__ __forceinline__ u64 ld_acquire(const u64 *p) {
