@@ -42,13 +42,11 @@ namespace ltlg {
 
 namespace {
 
-constexpr int OP_ANDOR_CLASS = 8;              // binary_row's class of & and | (the operator is a runtime value)
 constexpr int ENTRY_CACHE = 256;               // item starts of a plan's first entries kept in shared memory
 constexpr int NWARPS = LEVEL_THREADS / 32;
 constexpr int NCONS = NWARPS - 1;              // consumer warps per CTA
 static_assert(NCONS == LEVEL_CONSUMERS, "consumer warps");
 constexpr unsigned long long SPLIT_MAX_CANDS = 8192;  // levels below: rows split over warps (8k, 64k, 512k measured)
-constexpr int WU = 1;  // chunks per lane loaded per round of a claim's write sweep (2 and 4 measured slower)
 
 constexpr u64 PIPE_WAIT_NS = 30000000000ull;   // a consumer's wait for the producer (beyond every producer bound)
 constexpr u64 EMPTY_WAIT_NS = 10000000000ull;  // the producer's wait for the consumers to leave a slot
@@ -66,17 +64,18 @@ struct Slot {
     unsigned rows_done;
     unsigned evals;           // candidates evaluated in this item
     int kind;                 // ENT_*; 0 = the producer has ended
-    int op;                   // binary: OP_AND / OP_OR / OP_U; unary: opmask
+    int op;                   // binary: OP_AND / OP_OR / OP_U (fused: OP_AND); unary: opmask
     int nl;                   // binary: left rows in the tile
     int nrows;                // rows of the item
     int pos;                  // the entry's block position
-    int upos[4];              // unary: block position of each slot operator
+    int upos[4];              // unary: block position of each slot operator; fused binary: of & | U
     int cost;
     int check_only;
     int stop;                 // remaining rows are skipped (a find at or before this entry)
     int inst;                 // the item's instance (index into Launch::args)
     int trace_first;          // the producer's first item of this plan (level stamps)
-    int split;                // units per row: 1, or (a small level) one per left row / unary operator
+    int split;                // units per row (left groups of the tile; a small level's unary operators)
+    int lefts;                // binary: left rows of a unit
     int units;                // nrows * split: what the consumers take
     int overflowed;           // the cache had overflowed when the item was claimed (or a claim here
                               // overflowed): the rows' new CSs take no hash slots
@@ -86,26 +85,66 @@ struct Slot {
 
 // ---------------------------------------------------------------- candidate generators
 // pre(c) loads everything of chunk c that the set's candidates read from global memory
-// (binary: the right row; unary: the source row and the word metadata); word(t, c, pre) gives
-// words 2c, 2c+1 of candidate t from it (and the shared-memory tile).  A sweep that stores
-// words can so issue the loads of several chunks before its first store.
-template <int OPC>
-struct BinGen {
+// (binary: the right row; unary: the source row and the word metadata); each(c, pre, m, f) calls
+// f(t, words 2c and 2c + 1 of candidate t) for the candidates in mask m (the same in every lane),
+// loading each left row's chunk from the shared-memory tile once.
+
+// What a binary unit evaluates on each (left, right) pair: & | and both U orders; & and |; both U
+// orders; or one of & and |.
+enum { M_ALL = 0, M_AO = 1, M_U = 2, M_ONE = 3 };
+__host__ __device__ constexpr int mode_ops(int mode) { return mode == M_ALL ? 4 : mode == M_ONE ? 1 : 2; }
+// Operator of candidate o of a pair, and whether it is r U l (the pair's other order).
+__device__ __forceinline__ int mode_op(int mode, int o, int rop) {
+    return mode == M_ALL ? (o == 0 ? OP_AND : o == 1 ? OP_OR : OP_U)
+           : mode == M_AO ? (o == 0 ? OP_AND : OP_OR)
+           : mode == M_U  ? OP_U
+                          : rop;
+}
+__device__ __forceinline__ bool mode_swapped(int mode, int o) {
+    return (mode == M_ALL && o == 3) || (mode == M_U && o == 1);
+}
+
+template <int MODE, class F>
+__device__ __forceinline__ void pair_words(ulonglong2 l, ulonglong2 r, int rop, u32 m, F f) {
+    if (MODE == M_ALL || MODE == M_AO) {
+        if (m & 1u) f(0, l.x & r.x, l.y & r.y);
+        if (m & 2u) f(1, l.x | r.x, l.y | r.y);
+    }
+    if (MODE == M_ALL || MODE == M_U) {
+        constexpr int o = MODE == M_ALL ? 2 : 0;
+        const u64 ax = l.x | r.x, ay = l.y | r.y;
+        if (m & (1u << o)) f(o, row_until(ax, r.x), row_until(ay, r.y));            // l U r
+        if (m & (2u << o)) f(o + 1, row_until(ax, l.x), row_until(ay, l.y));        // r U l
+    }
+    if (MODE == M_ONE) {
+        if (rop == OP_AND)
+            f(0, l.x & r.x, l.y & r.y);
+        else
+            f(0, l.x | r.x, l.y | r.y);
+    }
+}
+
+template <int MODE, int NL>
+struct PairGen {
     using Pre = ulonglong2;
+    static constexpr int OPS = mode_ops(MODE);
     const ulonglong2 *left;   // shared-memory tile, row stride nch
     const ulonglong2 *right;  // global right row
     int nch;
     int rop;
     __device__ __forceinline__ Pre pre(int c) const { return __ldcg(right + c); }
-    __device__ __forceinline__ ulonglong2 word(int t, int c, ulonglong2 r) const {
-        if (OPC == OP_U) {
-            const ulonglong2 l = left[(t >> 1) * nch + c];
-            const u64 ax = l.x | r.x, ay = l.y | r.y;
-            if (t & 1) return make_ulonglong2(row_until(ax, l.x), row_until(ay, l.y));
-            return make_ulonglong2(row_until(ax, r.x), row_until(ay, r.y));
+    template <class F>
+    __device__ __forceinline__ void each(int c, const Pre &r, u32 m, F f) const {
+#pragma unroll
+        for (int u = 0; u < NL; ++u) {
+            const u32 mu = (m >> (u * OPS)) & ((1u << OPS) - 1u);
+            if (mu) pair_words<MODE>(left[u * nch + c], r, rop, mu, [&](int o, u64 x, u64 y) { f(u * OPS + o, x, y); });
         }
-        const ulonglong2 l = left[t * nch + c];
-        return rop == OP_AND ? make_ulonglong2(l.x & r.x, l.y & r.y) : make_ulonglong2(l.x | r.x, l.y | r.y);
+    }
+    __device__ __forceinline__ ulonglong2 word(int t, int c, const Pre &r) const {  // candidate t, any lane's t
+        ulonglong2 w = make_ulonglong2(0, 0);
+        pair_words<MODE>(left[(t / OPS) * nch + c], r, rop, 1u << (t % OPS), [&](int, u64 x, u64 y) { w = make_ulonglong2(x, y); });
+        return w;
     }
 };
 
@@ -118,6 +157,13 @@ struct UnGen {
     const ulonglong2 *src;
     const ulonglong2 *meta;
     __device__ __forceinline__ Pre pre(int c) const { return UnPre{__ldcg(meta + c), __ldcg(src + c)}; }
+    template <class F>
+    __device__ __forceinline__ void each(int, const Pre &p, u32 m, F f) const {
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+            if ((m >> t) & 1u)
+                f(t, row_unary(unary_slot_op(t), p.s.x, p.m.x & LENMASK), row_unary(unary_slot_op(t), p.s.y, p.m.y & LENMASK));
+    }
     __device__ __forceinline__ ulonglong2 word(int t, int, const Pre &p) const {
         const int op = unary_slot_op(t);
         return make_ulonglong2(row_unary(op, p.s.x, p.m.x & LENMASK), row_unary(op, p.s.y, p.m.y & LENMASK));
@@ -304,26 +350,16 @@ __device__ __forceinline__ void resolve(const InstArgs &A, InstCtl *C, int cost,
             if (lane == leader) base = atomicAdd(&C->row_count, (u64)__popc(cm));
             base = __shfl_sync(FULL, base, leader);
             const u64 cap = (u64)A.cap_rows;
-            // WU chunks per lane are loaded before any of their words is stored: the stores go
-            // to the same cache as the loads, so the compiler keeps them in program order
-            for (int c0 = lane; c0 < nch; c0 += 32 * WU) {
-                typename Gen::Pre pv[WU];
+            ulonglong2 *out[NC];
+            u32 wm = 0;  // the claims that found a row
 #pragma unroll
-                for (int u = 0; u < WU; ++u)
-                    if (c0 + 32 * u < nch) pv[u] = g.pre(c0 + 32 * u);
-#pragma unroll
-                for (int u = 0; u < WU; ++u) {
-                    const int c = c0 + 32 * u;
-                    if (c >= nch) break;
-#pragma unroll
-                    for (int t = 0; t < NC; ++t) {
-                        if ((cm >> t) & 1u) {
-                            const u64 row = base + __popc(cm & ((1u << t) - 1u));
-                            if (row < cap) reinterpret_cast<ulonglong2 *>(A.cache + row * pitch)[c] = g.word(t, c, pv[u]);
-                        }
-                    }
-                }
+            for (int t = 0; t < NC; ++t) {
+                const u64 row = base + __popc(cm & ((1u << t) - 1u));
+                out[t] = reinterpret_cast<ulonglong2 *>(A.cache + row * pitch);
+                if (((cm >> t) & 1u) && row < cap) wm |= 1u << t;
             }
+            for (int c = lane; c < nch; c += 32)
+                g.each(c, g.pre(c), wm, [&](int t, u64 x, u64 y) { out[t][c] = make_ulonglong2(x, y); });
             const u64 myrow = base + __popc(cm & ((1u << lane) - 1u));
             if (A.lstats) count_row_stats(A.lstats + (u64)cost * LSTATS, state == S_CLAIM && myrow < cap, anyp, anyn, lane);
             if (state == S_CLAIM && myrow < cap) {
@@ -368,24 +404,25 @@ __device__ __forceinline__ void resolve(const InstArgs &A, InstCtl *C, int cost,
         if (A.key_mode == KEY_EXACT) {
             const u32 vm = __ballot_sync(FULL, state == S_VERIFY);
             if (vm) {
-                u32 diff = 0;
+                u32 diffs[NC];
                 const u32 myv = (u32)vrow;
                 const ulonglong2 *vr[NC];
+#pragma unroll
+                for (int t = 0; t < NC; ++t) diffs[t] = 0;
 #pragma unroll
                 for (int t = 0; t < NC; ++t)
                     vr[t] = reinterpret_cast<const ulonglong2 *>(A.cache + (u64)__shfl_sync(FULL, myv, t) * pitch);
 #pragma unroll 1
                 for (int c = lane; c < nch; c += 32) {
-                    const auto p = g.pre(c);
-#pragma unroll
-                    for (int t = 0; t < NC; ++t) {
-                        if ((vm >> t) & 1u) {
-                            const ulonglong2 a = g.word(t, c, p);
-                            const ulonglong2 b = __ldcg(vr[t] + c);
-                            diff |= (u32)((a.x != b.x) | (a.y != b.y)) << t;
-                        }
-                    }
+                    g.each(c, g.pre(c), vm, [&](int t, u64 x, u64 y) {
+                        const ulonglong2 b = __ldcg(vr[t] + c);
+                        const u64 d = (x ^ b.x) | (y ^ b.y);
+                        diffs[t] |= hi32(d) | (u32)d;
+                    });
                 }
+                u32 diff = 0;
+#pragma unroll
+                for (int t = 0; t < NC; ++t) diff |= diffs[t] ? 1u << t : 0u;
                 const u32 anydiff = __reduce_or_sync(FULL, diff);
                 if (state == S_VERIFY) {
                     if ((anydiff >> lane) & 1u) {
@@ -467,14 +504,21 @@ __device__ __forceinline__ void finish(const InstArgs &A, InstCtl *C, Slot &sl, 
 }
 
 // ---------------------------------------------------------------- rows
-// Binary row: right row r (at R) against the slot's tile of TLP left rows (U: both orders of
-// each pair, TL = 2 TLP candidates; & and |: TL = TLP).  Chunks are 16 bytes (two words); two
-// are in flight per lane.  Positives are the first npos words, so acceptance needs no metadata.
-template <int OPC, int TL, int HK>
-__device__ __forceinline__ void binary_row(const InstArgs &A, InstCtl *C, Slot &sl, const ulonglong2 *tile,
-                                           int nl, long long l_first, const ulonglong2 *R, long long r, int lane) {
-    constexpr int TLP = OPC == OP_U ? TL / 2 : TL;
-    constexpr int NC = TL;
+// Binary unit: right row r (at R) against nl left rows of the slot's tile (row l_first and up),
+// every operator of MODE on each pair: NL * mode_ops(MODE) candidates.  Chunks are 16 bytes (two
+// words); two are in flight per lane.  Positives are the first npos words, so acceptance needs no
+// metadata.
+//
+// The sweep is bound by integer issue (ALU and the wide multiply-add), so it is laid out to share
+// work: one load of the pair's chunks feeds every operator (& | l U r r U l share l | r), the
+// word keys advance by additions, and acceptance is one three-input logic operation a word.
+// Measured with one operator at a time against all of them on one load (whole learns, unit or
+// near-unit costs): 1000 traces to cost 8 1.35 -> 1.14 ms, 4000 traces 10.4 -> 8.9 ms, 512 small
+// instances in a batch 18.8 -> 14.2 ms.
+template <int MODE, int NL, int HK>
+__device__ __forceinline__ void binary_unit(const InstArgs &A, InstCtl *C, Slot &sl, const ulonglong2 *tile, int nl,
+                                            long long l_first, const ulonglong2 *R, long long r, int lane) {
+    constexpr int OPS = mode_ops(MODE), NC = NL * OPS;
     const int nch = A.pitch >> 1, npos = A.npos, n = A.n;
     const int rop = sl.op;
     u64 h[NC];
@@ -487,6 +531,7 @@ __device__ __forceinline__ void binary_row(const InstArgs &A, InstCtl *C, Slot &
     const bool stats = A.lstats != nullptr;
     u32 bp = 0, bn = 0;
     constexpr int CH = 2;  // right-row chunks in flight per lane
+    u64 k = (2ull * (u64)lane + 1ull) * WEYL;
     for (int c0 = lane; c0 < nch; c0 += 32 * CH) {
         ulonglong2 rvv[CH];
 #pragma unroll
@@ -497,55 +542,57 @@ __device__ __forceinline__ void binary_row(const InstArgs &A, InstCtl *C, Slot &
 #pragma unroll
         for (int u = 0; u < CH; ++u) {
             const int c = c0 + 32 * u;
-            if (c >= nch) continue;
-            const u64 k = (2ull * (u64)c + 1ull) * WEYL;
-            const ulonglong2 rv = rvv[u];
-            const u32 p0 = 2 * c < npos ? ROW_BIT0_HI : 0u, p1 = 2 * c + 1 < npos ? ROW_BIT0_HI : 0u;
-            const bool v0 = 2 * c < n, v1 = 2 * c + 1 < n;
-            auto take = [&](int t, u64 w0, u64 w1) {
-                h[t] += hw<HK>(w0, k, v0) + hw<HK>(w1, k + WEYL, v1);
-                fails[t] |= fails2(w0, w1, p0, p1);
-                if (stats) {
-                    bp |= pmiss2(w0, w1, p0, p1) << t;
-                    bn |= nhit2(w0, w1, p0, p1) << t;
-                }
-            };
+            if (c < nch) {
+                const u32 p0 = 2 * c < npos ? ROW_BIT0_HI : 0u, p1 = 2 * c + 1 < npos ? ROW_BIT0_HI : 0u;
+                const bool v0 = 2 * c < n, v1 = 2 * c + 1 < n;
 #pragma unroll
-            for (int t = 0; t < TLP; ++t) {
-                if (t < nl) {
-                    const ulonglong2 lv = tile[t * nch + c];
-                    if (OPC == OP_U) {
-                        const u64 ax = lv.x | rv.x, ay = lv.y | rv.y;
-                        take(2 * t, row_until(ax, rv.x), row_until(ay, rv.y));      // l U r
-                        take(2 * t + 1, row_until(ax, lv.x), row_until(ay, lv.y));  // r U l
-                    } else if (rop == OP_AND) {
-                        take(t, lv.x & rv.x, lv.y & rv.y);
-                    } else {
-                        take(t, lv.x | rv.x, lv.y | rv.y);
+                for (int q = 0; q < NL; ++q) {
+                    if (q < nl) {
+                        pair_words<MODE>(tile[q * nch + c], rvv[u], rop, (1u << OPS) - 1u, [&](int o, u64 w0, u64 w1) {
+                            const int t = q * OPS + o;
+                            h[t] += hw<HK>(w0, k, v0) + hw<HK>(w1, k + WEYL, v1);
+                            fails[t] |= fails2(w0, w1, p0, p1);
+                            if (stats) {
+                                bp |= pmiss2(w0, w1, p0, p1) << t;
+                                bn |= nhit2(w0, w1, p0, p1) << t;
+                            }
+                        });
                     }
                 }
             }
+            k += 64ull * WEYL;
         }
     }
-    const int cnt = OPC == OP_U ? 2 * nl : nl;
-    const u32 valid = cnt >= 32 ? FULL : ((1u << cnt) - 1u);
-    const BinGen<OPC> g{tile, R, nch, rop};
+    const int cnt = OPS * nl;
+    const u32 valid = (1u << cnt) - 1u;
+    const PairGen<MODE, NL> g{tile, R, nch, rop};
     finish<NC>(A, C, sl, g, h, fails, bp, bn, valid,
                [&](int t) {
-                   if (OPC == OP_U) {
-                       const u64 l = (u64)(l_first + (t >> 1));
-                       return (t & 1) ? pack_parent(OP_U, (u64)r, l) : pack_parent(OP_U, l, (u64)r);
-                   }
-                   return pack_parent(rop, (u64)(l_first + t), (u64)r);
+                   const u64 l = (u64)(l_first + t / OPS);
+                   const int o = t % OPS;
+                   return mode_swapped(MODE, o) ? pack_parent(OP_U, (u64)r, l)
+                                                : pack_parent(mode_op(MODE, o, rop), l, (u64)r);
                },
-               [&](int) { return sl.pos; },
+               [&](int t) {  // fused entries: upos[0] &, [1] |, [2] U
+                   const int o = t % OPS;
+                   return MODE == M_ALL ? sl.upos[min(o, 2)] : MODE == M_AO ? sl.upos[o] : sl.pos;
+               },
                [&](int t) -> u64 {  // the reference's thread index: (l - l0) * R + (r - r0); U: both orders
-                   const u64 l = (u64)(l_first + (OPC == OP_U ? (t >> 1) : t));
+                   const u64 l = (u64)(l_first + t / OPS);
                    const u64 tid = (l - (u64)sl.e_l0) * (u64)sl.e_R + ((u64)r - (u64)sl.e_r0);
-                   return OPC == OP_U ? 2 * tid + (u64)(t & 1) : tid;
+                   const int o = t % OPS;
+                   return mode_op(MODE, o, rop) == OP_U ? 2 * tid + (u64)mode_swapped(MODE, o) : tid;
                },
                lane);
     if (lane == 0) atomicAdd(&sl.evals, (unsigned)cnt);
+}
+
+// Left rows a unit of each mode takes: tiles of 2 and 4 rows make units of 4 candidates (a tile of
+// 2 has two single-operator ones), tiles of 8 units of 8.
+template <int TL>
+__host__ __device__ constexpr int unit_lefts(int mode) {
+    constexpr int NC = TL == 8 ? 8 : 4;
+    return mode == M_ONE ? (TL < NC ? TL : NC) : NC / mode_ops(mode);
 }
 
 // Unary row: every operator of the slot's mask on source row s (at src; one load of each chunk).
@@ -560,6 +607,7 @@ __device__ __forceinline__ void unary_row(const InstArgs &A, InstCtl *C, Slot &s
     const bool stats = A.lstats != nullptr;
     u32 bp = 0, bn = 0;
     constexpr int CH = 2;  // source-row chunks in flight per lane
+    u64 k = (2ull * (u64)lane + 1ull) * WEYL;
     for (int c0 = lane; c0 < nch; c0 += 32 * CH) {
         ulonglong2 sv[CH], mv[CH];
 #pragma unroll
@@ -574,7 +622,6 @@ __device__ __forceinline__ void unary_row(const InstArgs &A, InstCtl *C, Slot &s
         for (int u = 0; u < CH; ++u) {
             const int c = c0 + 32 * u;
             if (c >= nch) continue;
-            const u64 k = (2ull * (u64)c + 1ull) * WEYL;
             const u32 p0 = 2 * c < npos ? ROW_BIT0_HI : 0u, p1 = 2 * c + 1 < npos ? ROW_BIT0_HI : 0u;
             const bool v0 = 2 * c < n, v1 = 2 * c + 1 < n;
             const u64 m0 = mv[u].x & LENMASK, m1 = mv[u].y & LENMASK;
@@ -591,6 +638,7 @@ __device__ __forceinline__ void unary_row(const InstArgs &A, InstCtl *C, Slot &s
                     }
                 }
             }
+            k += 64ull * WEYL;
         }
     }
     const u32 valid = (u32)(mask & 15);
@@ -604,14 +652,33 @@ __device__ __forceinline__ void unary_row(const InstArgs &A, InstCtl *C, Slot &s
 // ---------------------------------------------------------------- planner (one warp)
 __device__ __forceinline__ long long ls_at(const InstArgs &A, int k) { return __ldcg(A.ls + k); }
 
+// Level starts as the planning warp reads them: for levels up to 62 one load fills two registers a
+// lane and every later look-up is a shuffle (all lanes take part), beyond that each is a load.
+struct Levels {
+    long long a, b;  // ls[lane], ls[lane + 32]
+    int c, c1;
+    bool regs;
+};
+__device__ __forceinline__ Levels load_levels(const InstArgs &A, int c, int lane) {
+    Levels v;
+    v.c = c;
+    v.c1 = A.cf[0];
+    v.regs = c < 63;
+    v.a = lane <= c ? ls_at(A, lane) : 0ll;
+    v.b = lane + 32 <= c ? ls_at(A, lane + 32) : 0ll;
+    return v;
+}
+__device__ __forceinline__ long long level_start(const InstArgs &A, const Levels &v, int k) {
+    if (!v.regs) return ls_at(A, k);
+    const long long x = __shfl_sync(FULL, v.a, k & 31), y = __shfl_sync(FULL, v.b, k & 31);
+    return k >= 32 ? y : x;
+}
 // Rows of cost k < c: [lo, hi); empty outside c1 .. c - 1.
-__device__ __forceinline__ void level_range(const InstArgs &A, int k, int c, long long &lo, long long &hi) {
-    if (k < A.cf[0] || k >= c) {
-        lo = hi = 0;
-        return;
-    }
-    lo = ls_at(A, k);
-    hi = ls_at(A, k + 1);
+__device__ __forceinline__ void level_range(const InstArgs &A, const Levels &v, int k, long long &lo, long long &hi) {
+    const bool in = k >= v.c1 && k < v.c;
+    const long long x = level_start(A, v, in ? k : 0), y = level_start(A, v, in ? k + 1 : 0);
+    lo = in ? x : 0;
+    hi = in ? y : 0;
 }
 
 __device__ __forceinline__ void store_entry(Entry *dst, const Entry &e) {
@@ -621,49 +688,29 @@ __device__ __forceinline__ void store_entry(Entry *dst, const Entry &e) {
     for (int w = 0; w < (int)(sizeof(Entry) / 8); ++w) __stcg(d + w, s[w]);
 }
 
-// The binary blocks of operator op (cost cop) of level c, in the reference's split order
-// (i = c1 .. (c - cop) / 2 over non-empty levels i and j = c - i - cop): written as entries
-// from queue index *eidx and positions from *pos.  Returns the candidates of this lane's blocks.
-__device__ u64 plan_binary(const InstArgs &A, int c, int op, int ne_count, int ne_lane, int &pos, int &eidx,
-                           u64 &units, int lane) {
-    const int cop = A.cf[op + 1], c1 = A.cf[0];
-    const int tl = op == OP_U ? max(1, A.tile / 2) : A.tile;
-    u64 cand = 0;
-    if (c - cop < 2 * c1) return 0;
+// The splits of a binary operator of cost cop in level c, in the reference's order (i = c1 ..
+// (c - cop) / 2 over non-empty levels i and j = c - i - cop): f(exists, rank, i, left rows, right
+// rows), a lane per split; returns how many there are.  One warp.
+template <class F>
+__device__ __forceinline__ int each_split(const InstArgs &A, const Levels &v, int cop, int ne_count, int ne_lane, int lane,
+                                          F f) {
+    const int c = v.c;
+    int total = 0;
+    if (c - cop < 2 * v.c1) return 0;
     for (int base = 0; base < ne_count; base += 32) {
         const int q = base + lane;
         const int i = q < ne_count ? (base == 0 ? ne_lane : __ldcg(A.ne + q)) : 0;
-        const bool ok_i = q < ne_count && i >= c1 && 2 * i <= c - cop;
-        long long li = 0, hi_ = 0, lj = 0, hj = 0;
-        if (ok_i) {
-            level_range(A, i, c, li, hi_);
-            level_range(A, c - i - cop, c, lj, hj);
-        }
+        const bool ok_i = q < ne_count && i >= v.c1 && 2 * i <= c - cop;
+        long long li, hi_, lj, hj;
+        level_range(A, v, ok_i ? i : -1, li, hi_);
+        level_range(A, v, ok_i ? c - i - cop : -1, lj, hj);
         const bool ex = ok_i && hi_ > li && hj > lj;
         const u32 m = __ballot_sync(FULL, ex);
-        if (ex) {
-            const int rank = __popc(m & ((1u << lane) - 1u));
-            Entry e{};
-            e.kind = op == OP_U ? ENT_U : ENT_ANDOR;
-            e.op = op;
-            e.pos = pos + rank;
-            for (int j = 0; j < 4; ++j) e.upos[j] = POS_NONE;
-            e.lcost = i;
-            e.rcost = c - i - cop;
-            e.l0 = li;
-            e.l1 = hi_;
-            e.r0 = lj;
-            e.r1 = hj;
-            e.cand = (u64)(op == OP_U ? 2 : 1) * (u64)(hi_ - li) * (u64)(hj - lj);
-            cand += e.cand;
-            units += (u64)((hi_ - li + tl - 1) / tl) * (u64)(hj - lj);
-            store_entry(A.entries + eidx + rank, e);
-        }
-        pos += __popc(m);
-        eidx += __popc(m);
+        f(ex, total + __popc(m & ((1u << lane) - 1u)), i, li, hi_, lj, hj);
+        total += __popc(m);
         if (__any_sync(FULL, q < ne_count && 2 * i > c - cop)) break;  // the list is sorted by cost
     }
-    return cand;
+    return total;
 }
 
 // Builds the plan of level c in the reference's block order (ltli6463.cu:1209-1440): ~, &
@@ -676,26 +723,20 @@ __device__ void plan_level(const InstArgs &A, InstCtl *C, int c, int lane) {
     const u64 found_key = __ldcg(&C->found_key);  // loaded early: nothing changes it while planning
     // the first 32 non-empty levels, one per lane, for all three binary operators
     const int ne_lane = lane < ne_count ? __ldcg(A.ne + lane) : 0;
+    const Levels lev = load_levels(A, c, lane);
     // unary operators: lane j < 4 looks at slot operator j
-    bool uex = false;
+    const int uop = unary_slot_op(lane & 3), uk = c - A.cf[uop + 1];
+    bool uok = lane < 4 && uk >= c1;
+    if (uop == OP_NEG) uok = lane < 4 && ((A.neg_type == 1 && uk >= c1) || (A.neg_type == 2 && uk == c1));
     long long ulo = 0, uhi = 0;
-    int uk = 0;
-    if (lane < 4) {
-        const int op = unary_slot_op(lane);
-        uk = c - A.cf[op + 1];
-        bool ok = uk >= c1;
-        if (op == OP_NEG) ok = (A.neg_type == 1 && uk >= c1) || (A.neg_type == 2 && uk == c1);
-        if (ok) level_range(A, uk, c, ulo, uhi);
-        uex = ok && uhi > ulo;
-    }
+    level_range(A, lev, uok ? uk : -1, ulo, uhi);
+    const bool uex = uhi > ulo;
     const u32 um = __ballot_sync(FULL, uex) & 15u;
     long long lo4[4], hi4[4];
-    int k4[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         lo4[j] = __shfl_sync(FULL, ulo, j);
         hi4[j] = __shfl_sync(FULL, uhi, j);
-        k4[j] = __shfl_sync(FULL, uk, j);
     }
     // unary entries: one per distinct source range (fused) or per operator
     const bool fuse = !(A.plan_flags & PLAN_UNFUSED);
@@ -707,16 +748,65 @@ __device__ void plan_level(const InstArgs &A, InstCtl *C, int c, int lane) {
             if (group[q] >= 0 && lo4[q] == lo4[j] && hi4[q] == hi4[j]) group[j] = group[q];
         if (group[j] < 0) group[j] = nu++;
     }
-    // positions in the reference's order, binary entries after the unary ones in the queue
-    int pos = 0, eidx = nu;
+    // Binary operators of equal cost have the same splits, so one entry can run them on one load
+    // of each operand pair: & | U (the unit costs), or & and |.  Per-block runs and the learned
+    // order keep one entry per block.
+    const bool fuse2 = !(A.plan_flags & (PLAN_UNFUSED | PLAN_LEARNED)) && A.cf[OP_AND + 1] == A.cf[OP_OR + 1];
+    const bool fuse3 = fuse2 && A.cf[OP_AND + 1] == A.cf[OP_U + 1];
+    auto nothing = [](bool, int, int, long long, long long, long long, long long) {};
+    const int na = each_split(A, lev, A.cf[OP_AND + 1], ne_count, ne_lane, lane, nothing);
+    const int no = fuse2 ? na : each_split(A, lev, A.cf[OP_OR + 1], ne_count, ne_lane, lane, nothing);
+    // positions in the reference's order: ~, & splits, | splits, X, F, G, U splits; the queue runs
+    // the binary entries after the unary ones
     int upos[4] = {POS_NONE, POS_NONE, POS_NONE, POS_NONE};
+    int pos = 0, eidx = nu;
     if (um & 1u) upos[0] = pos++;
-    u64 units_b = 0, units_u = 0;  // binary: (left tile, right row) pairs; unary: source rows
-    u64 cand = plan_binary(A, c, OP_AND, ne_count, ne_lane, pos, eidx, units_b, lane);
-    cand += plan_binary(A, c, OP_OR, ne_count, ne_lane, pos, eidx, units_b, lane);
+    const int pos_and = pos, pos_or = pos_and + na;
+    pos = pos_or + no;
     for (int j = 1; j < 4; ++j)
         if ((um >> j) & 1u) upos[j] = pos++;
-    cand += plan_binary(A, c, OP_U, ne_count, ne_lane, pos, eidx, units_b, lane);
+    const int pos_u = pos;
+    u64 units_b = 0, units_u = 0;  // binary: (left tile, right row) pairs; unary: source rows
+    u64 cand = 0;
+    auto binary = [&](int op, int kind, int first) {
+        const int cop = A.cf[op + 1];
+        const int k = each_split(A, lev, cop, ne_count, ne_lane, lane,
+                                 [&](bool ex, int rank, int i, long long l0, long long l1, long long r0, long long r1) {
+            if (!ex) return;
+            Entry e{};
+            e.kind = kind;
+            e.op = op;
+            e.pos = first + rank;
+            e.upos[0] = first + rank;
+            e.upos[1] = kind == ENT_ALL || kind == ENT_AO ? pos_or + rank : POS_NONE;
+            e.upos[2] = kind == ENT_ALL ? pos_u + rank : POS_NONE;
+            e.upos[3] = POS_NONE;
+            e.lcost = i;
+            e.rcost = c - i - cop;
+            e.l0 = l0;
+            e.l1 = l1;
+            e.r0 = r0;
+            e.r1 = r1;
+            const u64 per_pair = kind == ENT_ALL ? 4 : kind == ENT_ONE ? 1 : 2;
+            e.cand = per_pair * (u64)(l1 - l0) * (u64)(r1 - r0);
+            cand += e.cand;
+            units_b += (u64)((l1 - l0 + A.tile - 1) / A.tile) * (u64)(r1 - r0);
+            store_entry(A.entries + eidx + rank, e);
+        });
+        eidx += k;
+        return k;
+    };
+    if (fuse3) {
+        pos += binary(OP_AND, ENT_ALL, pos_and);
+    } else {
+        if (fuse2) {
+            binary(OP_AND, ENT_AO, pos_and);
+        } else {
+            binary(OP_AND, ENT_ONE, pos_and);
+            binary(OP_OR, ENT_ONE, pos_or);
+        }
+        pos += binary(OP_U, ENT_U, pos_u);
+    }
     if (lane == 0) {
         for (int g = 0; g < nu; ++g) {
             Entry e{};
@@ -728,7 +818,7 @@ __device__ void plan_level(const InstArgs &A, InstCtl *C, int c, int lane) {
                 e.opmask |= 1 << j;
                 e.upos[j] = upos[j];
                 e.pos = min(e.pos, upos[j]);
-                e.lcost = k4[j];
+                e.lcost = c - A.cf[unary_slot_op(j) + 1];
                 e.r0 = lo4[j];
                 e.r1 = hi4[j];
                 e.cand += (u64)(hi4[j] - lo4[j]);
@@ -768,9 +858,8 @@ __device__ void plan_level(const InstArgs &A, InstCtl *C, int c, int lane) {
             if (kind == ENT_UNARY) {
                 it = (r1 - r0 + ur - 1) / ur;
             } else {
-                const int tl = kind == ENT_U ? max(1, A.tile / 2) : A.tile;
                 tiles_r = (r1 - r0 + rc - 1) / rc;
-                it = ((l1 - l0 + tl - 1) / tl) * tiles_r;
+                it = ((l1 - l0 + A.tile - 1) / A.tile) * tiles_r;
             }
         }
         // exclusive prefix of the item counts over the warp
@@ -1311,11 +1400,10 @@ __device__ __forceinline__ u32 fill_slot(Slot &sl, int inst, const Entry &e, lon
         sl.l_first = 0;
         return 0;
     }
-    const int tl = e.kind == ENT_U ? tile / 2 : tile;
     const long long ti = local / e.tiles_r, tr = local % e.tiles_r;
     sl.op = e.op;
-    sl.l_first = e.l0 + ti * tl;
-    sl.nl = (int)min((long long)tl, e.l1 - sl.l_first);
+    sl.l_first = e.l0 + ti * tile;
+    sl.nl = (int)min((long long)tile, e.l1 - sl.l_first);
     sl.row0 = e.r0 + tr * rc;
     sl.nrows = skip ? 1 : (int)min((long long)rc, e.r1 - sl.row0);
     return skip ? 0u : (u32)sl.nl * (u32)pitch * 8u;
@@ -1540,11 +1628,23 @@ __device__ void producer(const Launch &L, unsigned char *smem, u64 *tiles, int l
                                         pc.plan_items, skip, pc.a.pitch);
             sl.trace_first = pc.trace_first;
             sl.overflowed = ovf ? 1 : 0;
-            // a small level's rows are split into one unit per left row / unary operator, so
-            // more warps share its few rows (one warp's pass over a whole row is what such a
-            // level costs)
+            // units: a right row with unit_lefts of the tile's left rows; at a small level one left
+            // row / unary operator each, so more warps share its few rows (one warp's pass over a
+            // whole row is what such a level costs)
             int split = 1;
-            if (!skip && pc.split_small) split = sl.kind == ENT_UNARY ? __popc((unsigned)sl.op) : sl.nl;
+            sl.lefts = 1;
+            if (!skip) {
+                if (sl.kind == ENT_UNARY) {
+                    if (pc.split_small) split = __popc((unsigned)sl.op);
+                } else {
+                    if (!pc.split_small)
+                        sl.lefts = unit_lefts<TL>(sl.kind == ENT_ALL  ? M_ALL
+                                                  : sl.kind == ENT_AO ? M_AO
+                                                  : sl.kind == ENT_U  ? M_U
+                                                                      : M_ONE);
+                    split = (sl.nl + sl.lefts - 1) / sl.lefts;
+                }
+            }
             sl.split = max(1, split);
             sl.units = sl.nrows * sl.split;
             pc.trace_first = 0;
@@ -1576,9 +1676,9 @@ __device__ void producer(const Launch &L, unsigned char *smem, u64 *tiles, int l
     __syncwarp();
 }
 
-// The units of one slot a consumer warp takes, until the slot has none left: a unit is one row
-// of the item, or at a small level (split > 1) one left row of the tile against one right row,
-// or one unary operator on one source row.  Returns SLOT_CLOSE when this warp finished the
+// The units of one slot a consumer warp takes, until the slot has none left: a unit is one source
+// row under every operator of the item (at a small level under one), or one right row against a
+// group of the tile's left rows.  Returns SLOT_CLOSE when this warp finished the
 // level's last item, else SLOT_NEXT; closing the level (with the slot's arguments, before the
 // slot is released) is the caller's.
 enum { SLOT_NEXT = 0, SLOT_CLOSE = 1 };
@@ -1595,7 +1695,6 @@ __device__ __forceinline__ int take_rows(Slot &sl, int kind, const ulonglong2 *t
         if (idx == 0 && sl.trace_first && lane == 0)
             atomicCAS(A.level_ns + (u64)sl.cost * LEVEL_TRACE + LT_STARTED, 0ull, globaltimer());
         if (!*(volatile int *)&sl.stop) {
-            // a unit is a row, or with split one left row (binary) or one operator (unary) of it
             const int split = sl.split, part = (int)idx % split;
             const long long r = sl.row0 + (int)idx / split;
             const ulonglong2 *rp = reinterpret_cast<const ulonglong2 *>(A.cache + (u64)r * A.pitch);
@@ -1604,14 +1703,18 @@ __device__ __forceinline__ int take_rows(Slot &sl, int kind, const ulonglong2 *t
                 for (int q = 0; q < part && split > 1; ++q) mask &= mask - 1;  // the part-th operator
                 unary_row<HK>(A, C, sl, split > 1 ? (mask & -mask) : mask, rp, r, lane);
             } else {
-                const int nch = A.pitch >> 1;
-                const ulonglong2 *t0 = split > 1 ? tile + (u64)part * (u64)nch : tile;
-                const int nl = split > 1 ? 1 : sl.nl;
-                const long long lf = sl.l_first + (split > 1 ? part : 0);
-                if (kind == ENT_ANDOR)
-                    binary_row<OP_ANDOR_CLASS, TL, HK>(A, C, sl, t0, nl, lf, rp, r, lane);
+                const int nch = A.pitch >> 1, first = part * sl.lefts;
+                const ulonglong2 *t0 = tile + (u64)first * (u64)nch;
+                const int nl = min(sl.lefts, sl.nl - first);
+                const long long lf = sl.l_first + first;
+                if (kind == ENT_ALL)
+                    binary_unit<M_ALL, unit_lefts<TL>(M_ALL), HK>(A, C, sl, t0, nl, lf, rp, r, lane);
+                else if (kind == ENT_AO)
+                    binary_unit<M_AO, unit_lefts<TL>(M_AO), HK>(A, C, sl, t0, nl, lf, rp, r, lane);
+                else if (kind == ENT_U)
+                    binary_unit<M_U, unit_lefts<TL>(M_U), HK>(A, C, sl, t0, nl, lf, rp, r, lane);
                 else
-                    binary_row<OP_U, TL, HK>(A, C, sl, t0, nl, lf, rp, r, lane);
+                    binary_unit<M_ONE, unit_lefts<TL>(M_ONE), HK>(A, C, sl, t0, nl, lf, rp, r, lane);
             }
         }
         unsigned d = 0;

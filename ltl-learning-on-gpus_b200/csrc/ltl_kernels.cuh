@@ -63,17 +63,24 @@ constexpr u64 NO_FIND = ~0ull;         // InstCtl::found_key before any find
 constexpr int SEQ_SHIFT = 40;          // InstCtl::claimed = plan sequence << 40 | next item
 constexpr u64 ITEM_MASK = (1ull << SEQ_SHIFT) - 1;
 
-enum : int { ENT_UNARY = 1, ENT_ANDOR = 2, ENT_U = 3 };
+enum : int {
+    ENT_UNARY = 1,
+    ENT_ONE = 2,  // & or |
+    ENT_U = 3,    // both orders of U
+    ENT_ALL = 4,  // & | U of one split (equal operator costs)
+    ENT_AO = 5,   // & | of one split
+};
 
 // One entry of a level's plan, in queue order: one of the reference's (operator, split)
-// blocks, or (fused) every unary operator that reads the same source rows, so one load of a
-// source row serves all of them.
+// blocks, or (fused) every unary operator that reads the same source rows, or every binary
+// operator of equal cost on one split, so one load of the operands serves all of them.
 struct Entry {
-    int kind;            // ENT_UNARY, ENT_ANDOR, ENT_U
-    int op;              // binary: OP_AND / OP_OR / OP_U; unary: 0
+    int kind;            // ENT_*
+    int op;              // binary: OP_AND / OP_OR / OP_U (fused: OP_AND); unary: 0
     int opmask;          // unary: bit j = slot operator j (0 ~, 1 X, 2 F, 3 G)
-    int pos;             // position in the reference's block order (unary: the smallest of its operators)
-    int upos[4];         // unary: position of slot operator j's block, POS_NONE when absent
+    int pos;             // position in the reference's block order (fused: the smallest of its operators)
+    int upos[4];         // unary: position of slot operator j's block, POS_NONE when absent;
+                         // binary: of the &, |, U blocks it fuses (one block: its own first)
     int lcost, rcost;    // operand costs (unary: lcost is the operand's, rcost 0)
     long long l0, l1, r0, r1;  // binary: left rows [l0, l1) x right rows [r0, r1); unary: source rows [r0, r1)
     long long item0;     // first queue item of the entry
@@ -152,7 +159,7 @@ struct InstArgs {
     int cf[8];           // costs of p ~ & | X F G U
     int right_chunk_big, unary_rows_big;
     int small_rows;      // small levels: right rows (unary: source rows) per item
-    int tile;            // left rows staged per binary item (U: tile / 2 left rows)
+    int tile;            // left rows staged per binary item
     u32 gen;             // hash-set generation (1..255)
     int pad_;
     long long small_level;  // levels with fewer candidates size their items from the level (item_target)
@@ -235,7 +242,7 @@ struct Launch {
     BatchDev *batch;         // or null: a batch drains its pending instances through the slots
     int ninst;
     int persist;             // 1: after a level, plan and run the next one in the same launch
-    int tile;                // left rows staged per binary item (U: tile / 2 left rows, two candidates each)
+    int tile;                // left rows staged per binary item
     int stages;              // item slots in flight per CTA
     long long tile_bytes;    // shared-memory bytes of one slot's tile
 };

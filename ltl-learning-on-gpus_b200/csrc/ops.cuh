@@ -67,9 +67,10 @@ __device__ __forceinline__ u64 unary_bits(int op, u64 w, u64 m) {
 // candidates) 1.43 -> 1.35 ms, 4000 traces (602 thousand) 10.74 -> 10.45 ms.
 constexpr u32 ROW_BIT0_HI = 0x40000000u;  // position 0 in a row word's upper half
 
-__device__ __forceinline__ u64 row_until(u64 a, u64 y) {  // x U y, a = x | y
-    return ((a + y) ^ a ^ y) >> 1;
-}
+// x U y from a = x | y: with the sum s = a + y, a bit where a holds and y does not is the carry into
+// it inverted (s there is 1 ^ carry), and where y holds it is 1; so a & (y | ~s), two additions and
+// two three-input logic operations a word, without reading the carry out of the top.
+__device__ __forceinline__ u64 row_until(u64 a, u64 y) { return a & (y | ~(a + y)); }
 // F: every position at or before the last one where the operand holds: the bits at and above
 // the lowest set bit.  G: the positions after the last one (inside the trace) where it fails:
 // the operand's bits below the lowest set bit of z = ~w & m, all of them when z is 0 (the bits of
