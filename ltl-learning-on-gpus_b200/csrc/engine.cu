@@ -81,6 +81,33 @@ u64 host_fingerprint_exact(const uint64_t *w, int n, int pitch) {
     return host_fmix64(sum);
 }
 
+// A learn's upload: arguments, the level kernel's launch, the traces' record, then the relaxed keys'
+// bit placement (KEY_REF), the offsets and the steps.
+struct Up {
+    static constexpr size_t ARGS = 0, LAUNCH = 1024, IN = 1280, VAR = 1536;
+    size_t kmeta, offs, steps, bytes;
+    Up(int pitch, bool ref_keys, int n, long long nsteps, int width) {
+        kmeta = VAR;
+        offs = kmeta + (ref_keys ? (size_t)pitch * 4 : 0);
+        steps = offs + (size_t)(n + 1) * 4;
+        bytes = steps + (size_t)nsteps * (size_t)width;
+    }
+};
+static_assert(sizeof(InstArgs) <= Up::LAUNCH && sizeof(Launch) <= Up::IN - Up::LAUNCH && sizeof(StartIn) <= Up::VAR - Up::IN,
+              "upload layout");
+// A learn's results: the control block, the find's tree, level starts, candidates and stamps.
+constexpr int WALK_CAP = 256;
+struct Down {
+    static constexpr size_t CTL = 0, WALK = 1024, LS = WALK + (2 + 2 * WALK_CAP) * 8;
+    size_t lcands, lns, bytes;
+    explicit Down(long long ncost) {
+        lcands = LS + (size_t)ncost * 8;
+        lns = lcands + (size_t)ncost * 8;
+        bytes = lns + (size_t)ncost * LEVEL_TRACE * 8;
+    }
+};
+static_assert(sizeof(InstCtl) <= Down::WALK, "result layout");
+
 // Entries per level plan: 4 unary blocks and, per binary operator, a split per cost up to
 // max_cost / 2.
 long long entries_for(int max_cost) { return 4 + 3 * ((long long)max_cost / 2 + 2); }
@@ -93,14 +120,15 @@ struct ltlg_engine {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev_a = nullptr, ev_b = nullptr;
     // device buffers of the instance
-    DevBuf cache, parents, keys, prio, slots, wmeta, kmeta, ls, ne, lcands, lns, lstats, entries, fpar;
-    DevBuf ctl, args, launch, walk, snaps, scorer, scorer_params;
+    DevBuf cache, parents, keys, prio, slots, wmeta, ne, lstats, entries, fpar, snaps, scorer, scorer_params;
+    // what a learn sends down and what it reads back, each one block with one copy (layouts: Up, Down)
+    DevBuf up, down, h_up, h_down;
     // pinned host copies
-    DevBuf h_ctl, h_args, h_launch, h_walk, h_stage, h_ls, h_lcands, h_lns, h_ne, h_snaps, h_win, h_entries, h_fpar,
-        h_lstats;
+    DevBuf h_ctl, h_args, h_ne, h_snaps, h_win, h_entries, h_fpar, h_lstats;
     volatile u32 *cancel = nullptr;  // mapped host flag read by the planner
     void *cancel_dev = nullptr;
     bool has_scorer = false;
+    bool held = false;  // hold_slot: the next learn runs every level on the hash set in HBM
     u64 nslots = 0;
     u32 gen = 0;
     // last learn
@@ -110,6 +138,9 @@ struct ltlg_engine {
     long long tile_bytes = 0;
     std::vector<long long> level_start;
     std::string last_error;
+    InstArgs *args() const { return (InstArgs *)((char *)up.p + Up::ARGS); }
+    Launch *launch() const { return (Launch *)((char *)up.p + Up::LAUNCH); }
+    InstCtl *ctl() const { return (InstCtl *)((char *)down.p + Down::CTL); }
 };
 
 namespace {
@@ -199,14 +230,17 @@ void build_string(const std::map<u64, u64> &par, u64 row, u64 p, bool is_root, c
 }
 
 // Level-kernel geometry for rows of `pitch` words: the left tile (shrunk from `want` until at
-// least three item slots fit the shared memory) and the slots.  Returns false when not even one
-// slot of a 2-row tile fits.
+// least three item slots fit the shared memory) and the slots.  Wide rows (a tile of two rows) leave
+// room for the consumer warps' rings, and go down to one row where two slots do not fit.  Returns
+// false when not even one slot of a 1-row tile fits.
 bool geometry(int want, int pitch, int &tile, int &stages, long long &tile_bytes) {
-    constexpr long long BUDGET = 200 * 1024;  // dynamic shared memory for the slots' tiles
+    // dynamic shared memory for the slots' tiles, of an SM's 227 KB
+    constexpr long long BUDGET = 200 * 1024, WIDE = 215 * 1024 - level_ring_bytes(2);
     tile = want;
     while (tile > 2 && BUDGET / ((long long)tile * pitch * 8) < 3) tile /= 2;
+    if (tile == 2 && WIDE / ((long long)tile * pitch * 8) < 2) tile = 1;
     tile_bytes = (long long)tile * pitch * 8;
-    stages = (int)std::min<long long>(8, BUDGET / tile_bytes);
+    stages = (int)std::min<long long>(8, (tile <= 2 ? WIDE : BUDGET) / tile_bytes);
     return stages >= 1;
 }
 
@@ -298,14 +332,8 @@ LTLG_API int ltlg_engine_create(const ltlg_engine_config *cfg_in, ltlg_engine **
     if (err == cudaSuccess) err = ensure(e->slots, e->nslots * 8);
     if (err == cudaSuccess) err = cudaMemsetAsync(e->slots.p, 0, e->nslots * 8, e->stream);
     if (err == cudaSuccess) err = ensure(e->cache, (size_t)cfg.cache_bytes);
-    if (err == cudaSuccess) err = ensure(e->ctl, sizeof(InstCtl));
     if (err == cudaSuccess) err = ensure_host(e->h_ctl, sizeof(InstCtl));
-    if (err == cudaSuccess) err = ensure(e->args, sizeof(InstArgs));
     if (err == cudaSuccess) err = ensure_host(e->h_args, sizeof(InstArgs));
-    if (err == cudaSuccess) err = ensure(e->launch, sizeof(Launch));
-    if (err == cudaSuccess) err = ensure_host(e->h_launch, sizeof(Launch));
-    if (err == cudaSuccess) err = ensure(e->walk, (2 + 2 * 1024) * 8);
-    if (err == cudaSuccess) err = ensure_host(e->h_walk, (2 + 2 * 1024) * 8);
     if (err == cudaSuccess) {
         void *p = nullptr;
         err = cudaHostAlloc(&p, 64, cudaHostAllocMapped);
@@ -328,12 +356,11 @@ LTLG_API void ltlg_engine_destroy(ltlg_engine *e) {
     if (!e) return;
     cudaSetDevice(e->cfg.device);
     if (e->stream) cudaStreamSynchronize(e->stream);
-    for (DevBuf *b : {&e->cache, &e->parents, &e->keys, &e->prio, &e->slots, &e->wmeta, &e->kmeta, &e->ls, &e->ne, &e->lcands,
-                      &e->lns, &e->lstats, &e->entries, &e->fpar, &e->ctl, &e->args, &e->launch, &e->walk, &e->snaps,
-                      &e->scorer, &e->scorer_params})
+    for (DevBuf *b : {&e->cache, &e->parents, &e->keys, &e->prio, &e->slots, &e->wmeta, &e->ne, &e->lstats, &e->entries,
+                      &e->fpar, &e->snaps, &e->scorer, &e->scorer_params, &e->up, &e->down})
         if (b->p) cudaFree(b->p);
-    for (DevBuf *b : {&e->h_ctl, &e->h_args, &e->h_launch, &e->h_walk, &e->h_stage, &e->h_ls, &e->h_lcands, &e->h_lns,
-                      &e->h_ne, &e->h_snaps, &e->h_win, &e->h_entries, &e->h_fpar, &e->h_lstats})
+    for (DevBuf *b : {&e->h_ctl, &e->h_args, &e->h_ne, &e->h_snaps, &e->h_win, &e->h_entries, &e->h_fpar, &e->h_lstats,
+                      &e->h_up, &e->h_down})
         if (b->p) cudaFreeHost(b->p);
     if (e->cancel) cudaFreeHost((void *)e->cancel);
     for (cudaEvent_t ev : {e->ev_a, e->ev_b})
@@ -354,26 +381,20 @@ LTLG_API void ltlg_result_free(ltlg_result *r) {
 
 namespace {
 
-// Runs the level kernel once over the engine's instance and waits for it, with the learn's
-// time limit (the planner ends the search at the next level boundary once the cancel flag is set).
-cudaError_t run_levels(ltlg_engine *e, bool persist, int grid, double t0, double time_limit_s, LoopOut &o) {
-    Launch *hl = (Launch *)e->h_launch.p;
-    memset(hl, 0, sizeof(Launch));  // no batch: one instance
-    hl->args = (const InstArgs *)e->args.p;
-    hl->batch = nullptr;
-    hl->ninst = 1;
-    hl->persist = persist ? 1 : 0;
-    hl->tile = e->tile;
-    hl->stages = e->stages;
-    hl->tile_bytes = e->tile_bytes;
-    cudaStream_t st = e->stream;
-    cudaError_t err = cudaMemcpyAsync(e->launch.p, hl, sizeof(Launch), cudaMemcpyHostToDevice, st);
-    if (err != cudaSuccess) return err;
-    cudaEventRecord(e->ev_a, st);
-    err = launch_levels(*hl, (const Launch *)e->launch.p, grid, e->hk, st);
-    if (err != cudaSuccess) return err;
-    cudaEventRecord(e->ev_b, st);
-    ++o.launches;
+void fill_launch(const ltlg_engine *e, Launch &L, bool persist) {
+    memset(&L, 0, sizeof(Launch));  // no batch: one instance
+    L.args = e->args();
+    L.ninst = 1;
+    L.persist = persist ? 1 : 0;
+    L.tile = e->tile;
+    L.stages = e->stages;
+    L.tile_bytes = e->tile_bytes;
+}
+
+// Waits for ev_b, with the learn's time limit (the planner ends the search at the next level boundary
+// once the cancel flag is set), and adds the device time since ev_a.
+cudaError_t wait_levels(ltlg_engine *e, double t0, double time_limit_s, LoopOut &o) {
+    cudaError_t err;
     if (time_limit_s > 0) {
         while ((err = cudaEventQuery(e->ev_b)) == cudaErrorNotReady) {
             if (now_s() - t0 > time_limit_s) *e->cancel = 1u;
@@ -389,8 +410,23 @@ cudaError_t run_levels(ltlg_engine *e, bool persist, int grid, double t0, double
     return cudaSuccess;
 }
 
+// Runs the level kernel once over the open window of a host-driven level and waits for it.
+cudaError_t run_levels(ltlg_engine *e, int grid, double t0, LoopOut &o) {
+    Launch *hl = (Launch *)((char *)e->h_up.p + Up::LAUNCH);
+    fill_launch(e, *hl, false);
+    cudaStream_t st = e->stream;
+    cudaError_t err = cudaMemcpyAsync(e->launch(), hl, sizeof(Launch), cudaMemcpyHostToDevice, st);
+    if (err != cudaSuccess) return err;
+    cudaEventRecord(e->ev_a, st);
+    err = launch_levels(*hl, e->launch(), grid, e->hk, st);
+    if (err != cudaSuccess) return err;
+    cudaEventRecord(e->ev_b, st);
+    ++o.launches;
+    return wait_levels(e, t0, 0.0, o);
+}
+
 cudaError_t read_ctl(ltlg_engine *e, InstCtl *hc) {
-    cudaError_t err = cudaMemcpyAsync(hc, e->ctl.p, sizeof(InstCtl), cudaMemcpyDeviceToHost, e->stream);
+    cudaError_t err = cudaMemcpyAsync(hc, e->ctl(), sizeof(InstCtl), cudaMemcpyDeviceToHost, e->stream);
     if (err == cudaSuccess) err = cudaStreamSynchronize(e->stream);
     return err;
 }
@@ -400,9 +436,18 @@ cudaError_t open_window(ltlg_engine *e, u32 seq, long long lo, long long hi, int
     u64 *w = (u64 *)e->h_win.p + 2 * slot;
     w[0] = ((u64)seq << SEQ_SHIFT) | (u64)lo;
     w[1] = ((u64)seq << SEQ_SHIFT) | (u64)hi;
-    InstCtl *dc = (InstCtl *)e->ctl.p;
+    InstCtl *dc = e->ctl();
     cudaError_t err = cudaMemcpyAsync(&dc->limit, &w[1], 8, cudaMemcpyHostToDevice, e->stream);
     if (err == cudaSuccess) err = cudaMemcpyAsync(&dc->claimed, &w[0], 8, cudaMemcpyHostToDevice, e->stream);
+    return err;
+}
+
+// What host-driven levels (per-block runs, the on-the-fly regime, block labels) need besides.
+cudaError_t ensure_host_levels(ltlg_engine *e, long long cap_entries) {
+    cudaError_t err = ensure(e->snaps, (size_t)cap_entries * 8);
+    if (err == cudaSuccess) err = ensure_host(e->h_snaps, (size_t)cap_entries * 8);
+    if (err == cudaSuccess) err = ensure_host(e->h_win, (size_t)(2 * cap_entries + 2) * 8);
+    if (err == cudaSuccess) err = ensure_host(e->h_entries, (size_t)cap_entries * sizeof(Entry));
     return err;
 }
 
@@ -444,28 +489,21 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
     cudaError_t err = cudaSetDevice(e->cfg.device);
     if (err != cudaSuccess) return fail_cuda(e, err, res);
 
-    // Letters (ltli6463.cu:1100-1136): CS rows 0 .. nalpha-1; the first letter that
-    // separates the traces ends the search at cost c1.
+    // The first letter that separates the traces ends the search at cost c1 (ltli6463.cu:1100-1136):
+    // it holds at step 0 of every positive and of no negative.  The letters' rows are made on the device.
     const int pitch = std::max(4, (n + 3) & ~3);
-    std::vector<u64> letters((size_t)nalpha * pitch, 0ull);
-    int letter_hit = -1;
-    uint64_t all = 0;
-    for (int j = 0; j < nalpha; ++j) {
-        const uint32_t bit = 1u << (alpha[j] - 'a');
-        bool acc = true;
-        for (int i = 0; i < n; ++i) {
-            u64 w = 0;
-            for (int k = t->offsets[i]; k < t->offsets[i + 1]; ++k)
-                if (t->steps[k] & bit) w |= 1ull << (62 - (k - t->offsets[i]));
-            letters[(size_t)j * pitch + i] = w;
-            if (((w >> 62) != 0) != (i < npos)) acc = false;
-        }
-        all++;
-        if (acc && letter_hit < 0) {
-            letter_hit = j;
-            if (opt->stop_at_found) break;
-        }
+    uint32_t every = ~0u, some = 0u;
+    for (int i = 0; i < n; ++i) {
+        const uint32_t m = t->offsets[i + 1] > t->offsets[i] ? t->steps[t->offsets[i]] : 0u;
+        if (i < npos)
+            every &= m;
+        else
+            some |= m;
     }
+    int letter_hit = -1;
+    for (int j = 0; j < nalpha && letter_hit < 0; ++j)
+        if (((every & ~some) >> (alpha[j] - 'a')) & 1u) letter_hit = j;
+    uint64_t all = letter_hit >= 0 && opt->stop_at_found ? (uint64_t)letter_hit + 1 : (uint64_t)nalpha;
     const int max_cost = opt->max_cost;
     e->n = n;
     e->pitch = pitch;
@@ -502,8 +540,8 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
     long long tile_bytes = 0;
     if (!geometry(e->cfg.left_tile, pitch, tile, stages, tile_bytes)) return fail_status(res, LTLG_BAD_ARGS);
     const int hk = opt->key_mode == LTLG_KEY_HASH64 ? 1 : 0;
-    const size_t smem = level_kernel_smem(stages, tile_bytes);
-    const int per_sm = level_kernel_ctas_per_sm(hk, smem);
+    const size_t smem = level_kernel_smem(tile, stages, tile_bytes);
+    const int per_sm = level_kernel_ctas_per_sm(tile, hk, smem);
     if (per_sm < 1) return fail_status(res, LTLG_BAD_ARGS);
     e->tile = tile;
     e->stages = stages;
@@ -511,13 +549,26 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
     e->hk = hk;
     e->grid = e->num_sms * per_sm;
 
-    // Per-word metadata: length mask | positive flag; relaxed-key bit placement.
-    std::vector<u64> wmeta(pitch, 0ull);
-    std::vector<u32> kmeta(pitch, 0u);
-    for (int i = 0; i < n; ++i) {
-        const int ln = t->offsets[i + 1] - t->offsets[i];
-        wmeta[i] = row_lenmask(ln) | (i < npos ? (1ull << 63) : 0ull);
+    // the upload block; relaxed keys: each word's bit placement
+    const long long nsteps = (long long)t->offsets[n] - t->offsets[0];
+    // step masks go down in the fewest bytes that hold the span of the letters
+    int lo_bit = 25, hi_bit = 0;
+    for (char c : alpha) {
+        lo_bit = std::min(lo_bit, c - 'a');
+        hi_bit = std::max(hi_bit, c - 'a');
     }
+    const int width = hi_bit - lo_bit < 8 ? 1 : hi_bit - lo_bit < 16 ? 2 : 4;
+    const Up upl(pitch, ref_keys, n, nsteps, width);
+    if (upl.bytes > e->up.bytes) {
+        if ((err = cudaStreamSynchronize(e->stream)) != cudaSuccess) return fail_cuda(e, err, res);
+        const size_t want = std::max<size_t>(upl.bytes + upl.bytes / 4, 64 << 10);
+        if ((err = ensure(e->up, want)) != cudaSuccess || (err = ensure_host(e->h_up, want)) != cudaSuccess)
+            return fail_cuda(e, err, res);
+    }
+    char *hu = (char *)e->h_up.p;
+    char *du = (char *)e->up.p;
+    u32 *kmeta = (u32 *)(hu + upl.kmeta);
+    if (ref_keys) memset(kmeta, 0, (size_t)pitch * 4);
     int rlx_type = 0;
     if (ref_keys) {
         rlx_type = len_sum > 126 ? opt->rlx_unq_chk_type : 0;
@@ -545,52 +596,20 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
     if (opt->key_mode != LTLG_KEY_EXACT && (err = ensure(e->keys, (size_t)cap_rows * 16)) != cudaSuccess)
         return fail_cuda(e, err, res);
     if (ref_keys && (err = ensure(e->prio, (size_t)cap_rows * 8)) != cudaSuccess) return fail_cuda(e, err, res);
-    if ((err = ensure(e->wmeta, (size_t)pitch * 8)) != cudaSuccess) return fail_cuda(e, err, res);
-    if ((err = ensure(e->kmeta, (size_t)pitch * 4)) != cudaSuccess) return fail_cuda(e, err, res);
-    if ((err = ensure(e->ls, (size_t)ncost * 8)) != cudaSuccess) return fail_cuda(e, err, res);
-    if ((err = ensure(e->ne, (size_t)ncost * 4)) != cudaSuccess) return fail_cuda(e, err, res);
-    if ((err = ensure(e->lcands, (size_t)ncost * 8)) != cudaSuccess) return fail_cuda(e, err, res);
-    if ((err = ensure(e->lns, (size_t)ncost * LEVEL_TRACE * 8)) != cudaSuccess) return fail_cuda(e, err, res);
-    if ((err = ensure(e->lstats, (size_t)ncost * LSTATS * 8)) != cudaSuccess) return fail_cuda(e, err, res);
-    if ((err = ensure(e->entries, (size_t)(2 * cap_entries) * sizeof(Entry))) != cudaSuccess)
-        return fail_cuda(e, err, res);
-    if ((err = ensure(e->fpar, (size_t)cap_entries * 8)) != cudaSuccess) return fail_cuda(e, err, res);
-    if ((err = ensure(e->snaps, (size_t)cap_entries * 8)) != cudaSuccess) return fail_cuda(e, err, res);
-    if ((err = ensure_host(e->h_stage, std::max<size_t>((size_t)nalpha * pitch * 8, (size_t)pitch * 12))) !=
-            cudaSuccess ||
-        (err = ensure_host(e->h_ls, (size_t)ncost * 8)) != cudaSuccess ||
-        (err = ensure_host(e->h_lcands, (size_t)ncost * 8)) != cudaSuccess ||
-        (err = ensure_host(e->h_lns, (size_t)ncost * LEVEL_TRACE * 8)) != cudaSuccess ||
-        (err = ensure_host(e->h_snaps, (size_t)cap_entries * 8)) != cudaSuccess ||
-        (err = ensure_host(e->h_win, (size_t)(2 * cap_entries + 2) * 8)) != cudaSuccess ||
-        (err = ensure_host(e->h_entries, (size_t)cap_entries * sizeof(Entry))) != cudaSuccess)
+    const Down dl(ncost);
+    if ((err = ensure(e->wmeta, (size_t)pitch * 8)) != cudaSuccess || (err = ensure(e->ne, (size_t)ncost * 4)) != cudaSuccess ||
+        (err = ensure(e->lstats, (size_t)ncost * LSTATS * 8)) != cudaSuccess ||
+        (err = ensure(e->entries, (size_t)(2 * cap_entries) * sizeof(Entry))) != cudaSuccess ||
+        (err = ensure(e->fpar, (size_t)cap_entries * 8)) != cudaSuccess ||
+        (err = ensure(e->down, dl.bytes)) != cudaSuccess || (err = ensure_host(e->h_down, dl.bytes)) != cudaSuccess)
         return fail_cuda(e, err, res);
     cudaStream_t st = e->stream;
-    memcpy(e->h_stage.p, letters.data(), letters.size() * 8);
-    if ((err = cudaMemcpyAsync(e->cache.p, e->h_stage.p, letters.size() * 8, cudaMemcpyHostToDevice, st)) !=
-        cudaSuccess)
-        return fail_cuda(e, err, res);
-    if ((err = cudaStreamSynchronize(st)) != cudaSuccess) return fail_cuda(e, err, res);
-    memcpy(e->h_stage.p, wmeta.data(), (size_t)pitch * 8);
-    memcpy((char *)e->h_stage.p + (size_t)pitch * 8, kmeta.data(), (size_t)pitch * 4);
-    cudaMemcpyAsync(e->wmeta.p, e->h_stage.p, (size_t)pitch * 8, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(e->kmeta.p, (char *)e->h_stage.p + (size_t)pitch * 8, (size_t)pitch * 4, cudaMemcpyHostToDevice,
-                    st);
     // Hash-set generation: slots of older generations count as empty.
     if (++e->gen > 255) {
         cudaMemsetAsync(e->slots.p, 0, e->nslots * 8, st);
         e->gen = 1;
     }
-    cudaMemsetAsync(e->ls.p, 0, (size_t)ncost * 8, st);
-    cudaMemsetAsync(e->lcands.p, 0, (size_t)ncost * 8, st);
-    cudaMemsetAsync(e->lns.p, 0, (size_t)ncost * LEVEL_TRACE * 8, st);
-    if (want_stats) cudaMemsetAsync(e->lstats.p, 0, (size_t)ncost * LSTATS * 8, st);
     InstCtl *hc = (InstCtl *)e->h_ctl.p;
-    memset(hc, 0, sizeof(InstCtl));
-    hc->row_count = (u64)nalpha;
-    hc->found_key = NO_FIND;
-    hc->plan.cost = c1;
-    cudaMemcpyAsync(e->ctl.p, hc, sizeof(InstCtl), cudaMemcpyHostToDevice, st);
     *e->cancel = 0u;
 
     const bool per_block = opt->schedule == LTLG_SCHEDULE_PER_BLOCK;
@@ -630,36 +649,83 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
     A.prio = ref_keys ? (u64 *)e->prio.p : nullptr;
     A.slots = (u64 *)e->slots.p;
     A.wmeta = (const u64 *)e->wmeta.p;
-    A.kmeta = (const u32 *)e->kmeta.p;
-    A.ls = (long long *)e->ls.p;
+    A.kmeta = (const u32 *)(du + upl.kmeta);
+    A.ls = (long long *)((char *)e->down.p + Down::LS);
     A.ne = (int *)e->ne.p;
-    A.level_cands = (u64 *)e->lcands.p;
-    A.level_ns = (u64 *)e->lns.p;
+    A.level_cands = (u64 *)((char *)e->down.p + dl.lcands);
+    A.level_ns = (u64 *)((char *)e->down.p + dl.lns);
     A.lstats = want_stats ? (u64 *)e->lstats.p : nullptr;
     A.entries = (Entry *)e->entries.p;
     A.found_par = (u64 *)e->fpar.p;
-    A.ctl = (InstCtl *)e->ctl.p;
+    A.ctl = e->ctl();
     A.model = learned ? e->scorer.p : nullptr;
     // the planner reads the (mapped host) cancel flag at each level end only under a time limit
     A.cancel = opt->time_limit_s > 0 ? (const volatile u32 *)e->cancel_dev : nullptr;
-    const InstArgs *dA = (const InstArgs *)e->args.p;
-    cudaMemcpyAsync(e->args.p, ha, sizeof(InstArgs), cudaMemcpyHostToDevice, st);
-    if ((err = launch_insert_letters(dA, nalpha, hk, st)) != cudaSuccess) return fail_cuda(e, err, res);
+    // one copy down: arguments, launch, traces
     const bool persist = !per_block;
-    if ((err = launch_first_plan(dA, 1, persist ? 1 : 0, st)) != cudaSuccess) return fail_cuda(e, err, res);
-
+    const InstArgs *dA = e->args();
+    memcpy(hu + Up::ARGS, ha, sizeof(InstArgs));
+    Launch &L = *(Launch *)(hu + Up::LAUNCH);
+    fill_launch(e, L, persist);
+    StartIn &in = *(StartIn *)(hu + Up::IN);
+    memset(&in, 0, sizeof(in));
+    in.steps = du + upl.steps;
+    in.offs = (const int *)(du + upl.offs);
+    in.width = width;
+    for (int j = 0; j < nalpha; ++j) in.bit[j] = (char)(alpha[j] - 'a' - lo_bit);
+    {
+        int *o = (int *)(hu + upl.offs);
+        const int base = t->offsets[0];
+        for (int i = 0; i <= n; ++i) o[i] = t->offsets[i] - base;
+        const uint32_t *from = t->steps + base;
+        char *to = hu + upl.steps;
+        if (width == 1)
+            for (long long k = 0; k < nsteps; ++k) ((uint8_t *)to)[k] = (uint8_t)(from[k] >> lo_bit);
+        else if (width == 2)
+            for (long long k = 0; k < nsteps; ++k) ((uint16_t *)to)[k] = (uint16_t)(from[k] >> lo_bit);
+        else
+            for (long long k = 0; k < nsteps; ++k) ((uint32_t *)to)[k] = from[k] >> lo_bit;
+    }
+    const StartIn *din = (const StartIn *)(du + Up::IN);
+    if ((err = cudaMemcpyAsync(du, hu, upl.bytes, cudaMemcpyHostToDevice, st)) != cudaSuccess) return fail_cuda(e, err, res);
     LoopOut o;
-    o.launches = 2;
+    cudaEventRecord(e->ev_a, st);
+    const bool held = e->held;
+    e->held = false;
+    if (persist && !held && local_takes(A.key_mode, pitch)) {
+        // set-up and the small levels on one CTA
+        if ((err = launch_start(dA, din, hk, st)) != cudaSuccess) return fail_cuda(e, err, res);
+        o.launches = 1;
+    } else {
+        if ((err = launch_init(dA, din, pitch, st)) != cudaSuccess) return fail_cuda(e, err, res);
+        if ((err = launch_insert_letters(dA, nalpha, hk, st)) != cudaSuccess) return fail_cuda(e, err, res);
+        if ((err = launch_first_plan(dA, 1, persist ? 1 : 0, st)) != cudaSuccess) return fail_cuda(e, err, res);
+        o.launches = 3;
+    }
     o.last_cost = c1;
     int shortage = -1;
     bool last_round = false;
     uint64_t all_before = all;
-    InstCtl *dctl = (InstCtl *)e->ctl.p;
+    InstCtl *dctl = e->ctl();
     const double tl = opt->time_limit_s;
+    char *hd = (char *)e->h_down.p;
+    bool have_down = false;
     if (persist) {
-        // ---- every level in one launch, planned on the device
-        if ((err = run_levels(e, true, e->grid, t0, tl, o)) != cudaSuccess) return fail_cuda(e, err, res);
-        if ((err = read_ctl(e, hc)) != cudaSuccess) return fail_cuda(e, err, res);
+        // ---- every other level in one launch, planned on the device; then the find's tree, and one
+        // copy back
+        if ((err = launch_levels(L, e->launch(), e->grid, hk, st)) != cudaSuccess) return fail_cuda(e, err, res);
+        cudaEventRecord(e->ev_b, st);
+        u64 *dwalk = (u64 *)((char *)e->down.p + Down::WALK);
+        if ((err = launch_walk((const u64 *)e->parents.p, nalpha, 0, dctl, dwalk, WALK_CAP, st)) != cudaSuccess)
+            return fail_cuda(e, err, res);
+        o.launches += 2;
+        if ((err = cudaMemcpyAsync(hd, e->down.p, dl.bytes, cudaMemcpyDeviceToHost, st)) != cudaSuccess)
+            return fail_cuda(e, err, res);
+        if (tl > 0 && (err = wait_levels(e, t0, tl, o)) != cudaSuccess) return fail_cuda(e, err, res);
+        if ((err = cudaStreamSynchronize(st)) != cudaSuccess) return fail_cuda(e, err, res);
+        if (tl <= 0 && (err = wait_levels(e, t0, 0.0, o)) != cudaSuccess) return fail_cuda(e, err, res);
+        memcpy(hc, hd + Down::CTL, sizeof(InstCtl));
+        have_down = true;
         o.last_cost = std::max<int>(c1, (int)hc->last_cost);
         if (hc->status & ST_FATAL) {
             o.status = fatal_status(hc->status);
@@ -682,7 +748,7 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
     const bool host_levels = (per_block || o.on_the_fly) && o.status == LTLG_NOT_FOUND && !o.found;
     auto switch_on_the_fly = [&](int next_cost) -> cudaError_t {
         A.on_the_fly = 1;
-        cudaError_t x = cudaMemcpyAsync(e->args.p, ha, sizeof(InstArgs), cudaMemcpyHostToDevice, st);
+        cudaError_t x = cudaMemcpyAsync(e->args(), ha, sizeof(InstArgs), cudaMemcpyHostToDevice, st);
         if (x != cudaSuccess) return x;
         static const u32 zero = 0;
         x = cudaMemcpyAsync(&dctl->flags, &zero, 4, cudaMemcpyHostToDevice, st);
@@ -691,6 +757,7 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
         if (x == cudaSuccess) x = read_ctl(e, hc);
         return x;
     };
+    if (host_levels && (err = ensure_host_levels(e, cap_entries)) != cudaSuccess) return fail_cuda(e, err, res);
     if (host_levels && o.on_the_fly)
         if ((err = switch_on_the_fly((int)hc->last_cost + 1)) != cudaSuccess) return fail_cuda(e, err, res);
     if (host_levels) {
@@ -721,13 +788,13 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
                     if ((err = open_window(e, seq, E.item0, E.item0 + E.items, (int)q)) != cudaSuccess)
                         return fail_cuda(e, err, res);
                     const int grid = (int)std::max<long long>(1, std::min<long long>(E.items, e->grid));
-                    if ((err = run_levels(e, false, grid, t0, 0.0, o)) != cudaSuccess) return fail_cuda(e, err, res);
+                    if ((err = run_levels(e, grid, t0, o)) != cudaSuccess) return fail_cuda(e, err, res);
                 }
                 cudaMemcpyAsync(e->h_snaps.p, e->snaps.p, order.size() * 8, cudaMemcpyDeviceToHost, st);
             } else {
                 if ((err = open_window(e, seq, 0, hc->plan.items, 0)) != cudaSuccess) return fail_cuda(e, err, res);
                 const int grid = (int)std::max<long long>(1, std::min<long long>(hc->plan.items, e->grid));
-                if ((err = run_levels(e, false, grid, t0, 0.0, o)) != cudaSuccess) return fail_cuda(e, err, res);
+                if ((err = run_levels(e, grid, t0, o)) != cudaSuccess) return fail_cuda(e, err, res);
             }
             if ((err = read_ctl(e, hc)) != cudaSuccess) return fail_cuda(e, err, res);
             if (per_block) {
@@ -772,14 +839,19 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
     }
 
     // ---- level ranges, statistics, the reference's candidate count
-    cudaMemcpyAsync(e->h_ls.p, e->ls.p, (size_t)ncost * 8, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(e->h_lcands.p, e->lcands.p, (size_t)ncost * 8, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(e->h_lns.p, e->lns.p, (size_t)ncost * LEVEL_TRACE * 8, cudaMemcpyDeviceToHost, st);
-    if ((err = read_ctl(e, hc)) != cudaSuccess) return fail_cuda(e, err, res);
+    if (host_levels || !have_down) {
+        if ((err = launch_walk((const u64 *)e->parents.p, nalpha, 0, dctl, (u64 *)((char *)e->down.p + Down::WALK), WALK_CAP,
+                               st)) != cudaSuccess)
+            return fail_cuda(e, err, res);
+        ++o.launches;
+        cudaMemcpyAsync(hd, e->down.p, dl.bytes, cudaMemcpyDeviceToHost, st);
+        if ((err = cudaStreamSynchronize(st)) != cudaSuccess) return fail_cuda(e, err, res);
+        memcpy(hc, hd + Down::CTL, sizeof(InstCtl));
+    }
     const long long rows_final = std::min<long long>((long long)hc->row_count, cap_rows);
-    const long long *hls = (const long long *)e->h_ls.p;
-    const u64 *hlc = (const u64 *)e->h_lcands.p;
-    const u64 *hns = (const u64 *)e->h_lns.p;
+    const long long *hls = (const long long *)(hd + Down::LS);
+    const u64 *hlc = (const u64 *)(hd + dl.lcands);
+    const u64 *hns = (const u64 *)(hd + dl.lns);
     const bool found = o.found || hc->found != 0;
     const int found_cost = found ? (int)hc->found_cost : -1;
     const u64 found_word = hc->found;
@@ -848,14 +920,7 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
         res->cost = c1;
         res->status = LTLG_FOUND;
     } else if (found && found_word) {
-        const int wcap = 1024;
-        if ((err = launch_walk((const u64 *)e->parents.p, nalpha, found_word, (u64 *)e->walk.p, wcap, st)) !=
-            cudaSuccess)
-            return fail_cuda(e, err, res);
-        ++o.launches;
-        cudaMemcpyAsync(e->h_walk.p, e->walk.p, (2 + 2 * wcap) * 8, cudaMemcpyDeviceToHost, st);
-        if ((err = cudaStreamSynchronize(st)) != cudaSuccess) return fail_cuda(e, err, res);
-        const u64 *w = (const u64 *)e->h_walk.p;
+        const u64 *w = (const u64 *)(hd + Down::WALK);
         const u64 count = w[0], overflow = w[1];
         res->found_op = parent_op(found_word & ~(1ull << 63));
         if (overflow || count - 1 >= 200) {
@@ -938,14 +1003,15 @@ LTLG_API int ltlg_engine_label_blocks(ltlg_engine *e, const ltlg_traces *t, cons
     const int *cf = opt.cost_fun;
     cudaStream_t st = e->stream;
     InstArgs &A = *(InstArgs *)e->h_args.p;
-    const InstArgs *dA = (const InstArgs *)e->args.p;
+    const InstArgs *dA = e->args();
     const std::vector<long long> &ls = e->level_start;
     if ((int)ls.size() < c + 2) return rc;
     // Back to the start of level c: the rows of the lower levels stay, the list of non-empty
     // levels is cut at c, and level c is planned again with one entry per block, check-only
     // (every candidate's acceptance is tested, nothing stored).
     const long long ncost = (long long)e->max_cost + 3;
-    cudaError_t err = ensure_host(e->h_ne, (size_t)ncost * 4);
+    cudaError_t err = ensure_host_levels(e, entries_for(e->max_cost));
+    if (err == cudaSuccess) err = ensure_host(e->h_ne, (size_t)ncost * 4);
     if (err == cudaSuccess) err = ensure_host(e->h_lstats, (size_t)ncost * LSTATS * 8);
     if (err == cudaSuccess) err = cudaMemcpyAsync(e->h_ne.p, e->ne.p, (size_t)ncost * 4, cudaMemcpyDeviceToHost, st);
     InstCtl *hc = (InstCtl *)e->h_ctl.p;
@@ -966,8 +1032,8 @@ LTLG_API int ltlg_engine_label_blocks(ltlg_engine *e, const ltlg_traces *t, cons
     A.stop_at_found = 0;
     A.find_first = 0;
     A.max_cost = c;  // the window that finishes level c plans nothing after it
-    cudaMemcpyAsync(e->ctl.p, hc, sizeof(InstCtl), cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(e->args.p, &A, sizeof(InstArgs), cudaMemcpyHostToDevice, st);
+    cudaMemcpyAsync(e->ctl(), hc, sizeof(InstCtl), cudaMemcpyHostToDevice, st);
+    cudaMemcpyAsync(e->args(), &A, sizeof(InstArgs), cudaMemcpyHostToDevice, st);
     err = launch_plan_level(dA, c, st);
     if (err == cudaSuccess) err = read_ctl(e, hc);
     if (err != cudaSuccess) return fail_cuda(e, err, nullptr);
@@ -980,7 +1046,7 @@ LTLG_API int ltlg_engine_label_blocks(ltlg_engine *e, const ltlg_traces *t, cons
     if ((err = cudaStreamSynchronize(st)) != cudaSuccess) return fail_cuda(e, err, nullptr);
     // One window per block: the block's accepting candidates record themselves at its position.
     LoopOut o;
-    InstCtl *dctl = (InstCtl *)e->ctl.p;
+    InstCtl *dctl = e->ctl();
     static const u64 nofind = NO_FIND;
     for (int q = 0; q < ne; ++q) {
         const Entry &E = hent[q];
@@ -988,7 +1054,7 @@ LTLG_API int ltlg_engine_label_blocks(ltlg_engine *e, const ltlg_traces *t, cons
         if ((err = open_window(e, hc->seq, E.item0, E.item0 + E.items, q)) != cudaSuccess)
             return fail_cuda(e, err, nullptr);
         const int grid = (int)std::max<long long>(1, std::min<long long>(E.items, e->grid));
-        if ((err = run_levels(e, false, grid, now_s(), 0.0, o)) != cudaSuccess) return fail_cuda(e, err, nullptr);
+        if ((err = run_levels(e, grid, now_s(), o)) != cudaSuccess) return fail_cuda(e, err, nullptr);
     }
     cudaMemcpyAsync(e->h_fpar.p, e->fpar.p, (size_t)nbl * 8, cudaMemcpyDeviceToHost, st);
     if ((err = cudaStreamSynchronize(st)) != cudaSuccess) return fail_cuda(e, err, nullptr);
@@ -1072,8 +1138,9 @@ struct ltlg_batch {
     int num_sms = 0;
     cudaStream_t stream = nullptr;
     DevBuf cache, parents, keys, hslots, wmeta, kmeta, ls, ne, lcands, entries, fpar, ctl, args;
-    DevBuf bin, steps, offs, bout, cur, t0, bdev, launch;
-    DevBuf h_bin, h_steps, h_offs, h_bout, h_args, h_bdev, h_launch;
+    DevBuf bin, steps, offs, bout, cur, t0, bdev, launch, order;
+    DevBuf largs, lctl, lls, lne, llc, lpar, lmeta;  // per CTA of the small-level kernel (its rows are the slots' caches)
+    DevBuf h_bin, h_steps, h_offs, h_bout, h_args, h_bdev, h_launch, h_largs;
     std::vector<u32> gen;          // each slot's hash-set generation after the last call
     ltlg_engine *fallback = nullptr;
     std::vector<float> scorer;     // set_scorer's parameters, for the fallback engine
@@ -1137,9 +1204,10 @@ LTLG_API void ltlg_batch_destroy(ltlg_batch *b) {
     if (b->stream) cudaStreamSynchronize(b->stream);
     for (DevBuf *x : {&b->cache, &b->parents, &b->keys, &b->hslots, &b->wmeta, &b->kmeta, &b->ls, &b->ne, &b->lcands,
                       &b->entries, &b->fpar, &b->ctl, &b->args, &b->bin, &b->steps, &b->offs, &b->bout, &b->cur,
-                      &b->t0, &b->bdev, &b->launch})
+                      &b->t0, &b->bdev, &b->launch, &b->order, &b->largs, &b->lctl, &b->lls, &b->lne, &b->llc, &b->lpar,
+                      &b->lmeta})
         if (x->p) cudaFree(x->p);
-    for (DevBuf *x : {&b->h_bin, &b->h_steps, &b->h_offs, &b->h_bout, &b->h_args, &b->h_bdev, &b->h_launch})
+    for (DevBuf *x : {&b->h_bin, &b->h_steps, &b->h_offs, &b->h_bout, &b->h_args, &b->h_bdev, &b->h_launch, &b->h_largs})
         if (x->p) cudaFreeHost(x->p);
     if (b->stream) cudaStreamDestroy(b->stream);
     ltlg_engine_destroy(b->fallback);
@@ -1212,7 +1280,7 @@ LTLG_API int ltlg_batch_learn(ltlg_batch *b, const ltlg_traces *traces, int32_t 
         long long tile_bytes = 0;
         if (!geometry(b->cfg.left_tile, max_pitch, tile, stages, tile_bytes)) err = cudaErrorInvalidValue;
         const int per_sm =
-            err == cudaSuccess ? level_kernel_ctas_per_sm(hk, level_kernel_smem(stages, tile_bytes)) : 0;
+            err == cudaSuccess ? level_kernel_ctas_per_sm(tile, hk, level_kernel_smem(tile, stages, tile_bytes)) : 0;
         if (per_sm < 1 && err == cudaSuccess) err = cudaErrorInvalidConfiguration;
         const int grid = b->num_sms * std::max(per_sm, 1);
         // inputs: instance records, steps and offsets of every instance in one array each
@@ -1256,6 +1324,23 @@ LTLG_API int ltlg_batch_learn(ltlg_batch *b, const ltlg_traces *traces, int32_t 
         host(b->h_args, (size_t)K * sizeof(InstArgs));
         host(b->h_bdev, sizeof(BatchDev));
         host(b->h_launch, sizeof(Launch));
+        // The small levels of every instance run one CTA each, two CTAs an SM, before the slots take
+        // what is left; the CTAs' rows are cut out of the slots' caches, which are not in use then.  A
+        // handful of instances of long rows leaves most SMs idle that way: those go to the slots at once.
+        const bool local = err == cudaSuccess && min_pitch <= 1024 && (min_pitch <= 256 || nd >= b->num_sms);
+        const int lctas = std::min(nd, 2 * b->num_sms);
+        const long long lwords = (long long)K * cache_words / std::max(lctas, 1) & ~3ll;
+        if (local) {
+            dev(b->order, (size_t)nd * 4);
+            dev(b->largs, (size_t)lctas * sizeof(InstArgs));
+            dev(b->lctl, (size_t)lctas * sizeof(InstCtl));
+            dev(b->lls, (size_t)lctas * LOCAL_COSTS * 8);
+            dev(b->lne, (size_t)lctas * LOCAL_COSTS * 4);
+            dev(b->llc, (size_t)lctas * LOCAL_COSTS * 8);
+            dev(b->lpar, (size_t)lctas * LOCAL_ROWS * 8);
+            dev(b->lmeta, (size_t)lctas * max_pitch * 8);
+            host(b->h_largs, (size_t)lctas * sizeof(InstArgs));
+        }
         if (err == cudaSuccess) {
             BatchIn *bi = (BatchIn *)b->h_bin.p;
             u32 *hs = (u32 *)b->h_steps.p;
@@ -1325,6 +1410,8 @@ LTLG_API int ltlg_batch_learn(ltlg_batch *b, const ltlg_traces *traces, int32_t 
             D.t0 = (u64 *)b->t0.p;
             D.cache_words = cache_words;
             D.max_rows = max_rows;
+            D.order = local ? (int *)b->order.p : nullptr;
+            D.pending = local ? 0 : nd;
             D.count = nd;
             D.nslots = K;
             D.max_pitch = max_pitch;
@@ -1348,6 +1435,29 @@ LTLG_API int ltlg_batch_learn(ltlg_batch *b, const ltlg_traces *traces, int32_t 
             if (err == cudaSuccess) err = cudaMemsetAsync(b->ctl.p, 0, (size_t)K * sizeof(InstCtl), st);
             if (err == cudaSuccess) err = cudaMemcpyAsync(b->bdev.p, &D, sizeof(BatchDev), cudaMemcpyHostToDevice, st);
             if (err == cudaSuccess) err = cudaMemcpyAsync(b->launch.p, &L, sizeof(Launch), cudaMemcpyHostToDevice, st);
+            if (local) {
+                InstArgs *la = (InstArgs *)b->h_largs.p;
+                for (int q = 0; q < lctas; ++q) {
+                    InstArgs &A = la[q];
+                    A = ha[0];
+                    A.keys = nullptr;
+                    A.cache = (u64 *)b->cache.p + (size_t)q * lwords;
+                    A.parents = (u64 *)b->lpar.p + (size_t)q * LOCAL_ROWS;
+                    A.slots = nullptr;
+                    A.wmeta = (const u64 *)b->lmeta.p + (size_t)q * max_pitch;
+                    A.ls = (long long *)b->lls.p + (size_t)q * LOCAL_COSTS;
+                    A.ne = (int *)b->lne.p + (size_t)q * LOCAL_COSTS;
+                    A.level_cands = (u64 *)b->llc.p + (size_t)q * LOCAL_COSTS;
+                    A.entries = nullptr;
+                    A.found_par = nullptr;
+                    A.ctl = (InstCtl *)b->lctl.p + q;
+                }
+                const long long limit = LOCAL_LEVEL_WORK * std::max(1, std::min(LOCAL_BATCH_FACTOR, nd / b->num_sms * LOCAL_BATCH_FACTOR / 2));
+                if (err == cudaSuccess)
+                    err = cudaMemcpyAsync(b->largs.p, la, (size_t)lctas * sizeof(InstArgs), cudaMemcpyHostToDevice, st);
+                if (err == cudaSuccess)
+                    err = launch_batch_local((BatchDev *)b->bdev.p, (const InstArgs *)b->largs.p, lwords, limit, lctas, hk, st);
+            }
             if (err == cudaSuccess) err = launch_batch_start((BatchDev *)b->bdev.p, K, hk, st);
             if (err == cudaSuccess) err = launch_levels(L, (const Launch *)b->launch.p, grid, hk, st);
             if (err == cudaSuccess) err = cudaMemcpyAsync(b->h_bout.p, b->bout.p, bout_bytes, cudaMemcpyDeviceToHost, st);
@@ -1382,7 +1492,7 @@ LTLG_API int ltlg_batch_learn(ltlg_batch *b, const ltlg_traces *traces, int32_t 
             r->device_flags = o.device_flags;
             r->device_ms = (double)o.ns * 1e-6;
             r->seconds = wall;
-            r->launches = 2;
+            r->launches = local ? 3 : 2;
             std::string formula;
             if (o.letter >= 0 && o.letter < (int)alpha.size()) {
                 formula = std::string(1, alpha[o.letter]);
@@ -1460,7 +1570,9 @@ LTLG_API int ltlg_engine_hold_slot(ltlg_engine *e, const uint64_t *cs, int32_t n
     u64 *slot = (u64 *)e->slots.p + (fp & (e->nslots - 1));
     err = cudaMemcpyAsync(slot, &v, sizeof(v), cudaMemcpyHostToDevice, e->stream);
     if (err == cudaSuccess) err = cudaStreamSynchronize(e->stream);
-    return err == cudaSuccess ? 0 : fail_cuda(e, err, nullptr);
+    if (err != cudaSuccess) return fail_cuda(e, err, nullptr);
+    e->held = true;
+    return 0;
 }
 
 LTLG_API int ltlg_device_apply_op(int32_t op, const uint64_t *a, const uint64_t *b, const uint64_t *lenmask,

@@ -43,9 +43,6 @@ namespace ltlg {
 namespace {
 
 constexpr int ENTRY_CACHE = 256;               // item starts of a plan's first entries kept in shared memory
-constexpr int NWARPS = LEVEL_THREADS / 32;
-constexpr int NCONS = NWARPS - 1;              // consumer warps per CTA
-static_assert(NCONS == LEVEL_CONSUMERS, "consumer warps");
 constexpr unsigned long long SPLIT_MAX_CANDS = 8192;  // levels below: rows split over warps (8k, 64k, 512k measured)
 
 constexpr u64 PIPE_WAIT_NS = 30000000000ull;   // a consumer's wait for the producer (beyond every producer bound)
@@ -91,7 +88,7 @@ struct Slot {
 
 // What a binary unit evaluates on each (left, right) pair: & | and both U orders; & and |; both U
 // orders; or one of & and |.
-enum { M_ALL = 0, M_AO = 1, M_U = 2, M_ONE = 3 };
+enum { M_ALL = 0, M_AO = 1, M_U = 2, M_ONE = 3, M_UNARY = 4 };  // M_UNARY: no pair (csrc/local.cuh)
 __host__ __device__ constexpr int mode_ops(int mode) { return mode == M_ALL ? 4 : mode == M_ONE ? 1 : 2; }
 // Operator of candidate o of a pair, and whether it is r U l (the pair's other order).
 __device__ __forceinline__ int mode_op(int mode, int o, int rop) {
@@ -104,6 +101,14 @@ __device__ __forceinline__ bool mode_swapped(int mode, int o) {
     return (mode == M_ALL && o == 3) || (mode == M_U && o == 1);
 }
 
+// One candidate of a set, by what makes its words: the operator codes of the unary operators and
+// & |, and U in the order (left, right) or (right, left).  Unary operators read the row at `right`.
+enum { W_URL = 7 };  // r U l; l U r is OP_U
+struct Cand {
+    u32 left;                 // binary: the left row, in the shared-memory tile
+    const ulonglong2 *right;  // the right (unary: source) row
+    int wop;
+};
 template <int MODE, class F>
 __device__ __forceinline__ void pair_words(ulonglong2 l, ulonglong2 r, int rop, u32 m, F f) {
     if (MODE == M_ALL || MODE == M_AO) {
@@ -133,6 +138,10 @@ struct PairGen {
     int nch;
     int rop;
     __device__ __forceinline__ Pre pre(int c) const { return __ldcg(right + c); }
+    __device__ __forceinline__ Cand cand(int t) const {
+        const int o = t % OPS;
+        return Cand{smem_u32(left + (t / OPS) * nch), right, mode_swapped(MODE, o) ? (int)W_URL : mode_op(MODE, o, rop)};
+    }
     template <class F>
     __device__ __forceinline__ void each(int c, const Pre &r, u32 m, F f) const {
 #pragma unroll
@@ -157,6 +166,7 @@ struct UnGen {
     const ulonglong2 *src;
     const ulonglong2 *meta;
     __device__ __forceinline__ Pre pre(int c) const { return UnPre{__ldcg(meta + c), __ldcg(src + c)}; }
+    __device__ __forceinline__ Cand cand(int t) const { return Cand{0u, src, unary_slot_op(t & 3)}; }
     template <class F>
     __device__ __forceinline__ void each(int, const Pre &p, u32 m, F f) const {
 #pragma unroll
@@ -170,6 +180,102 @@ struct UnGen {
     }
 };
 
+// Sweeps over whole rows.  Lane l handles chunks l, l + 32, ... (16 bytes, two words).  What a sweep
+// reads from global memory goes through the warp's ring in shared memory: each lane copies its
+// own chunks ahead with cp.async and reads them back itself, so loads in flight cost no registers.
+// A stage of the ring holds two chunks per lane of each of NS rows; D stages.
+template <int NS, int D, class F>
+__device__ __forceinline__ void stream(const ulonglong2 *const (&src)[NS], int nch, u32 ring, int lane, F f) {
+    constexpr u32 CH = 512, STAGE = 2 * NS * CH;  // one chunk per lane, one stage
+    static_assert(D * STAGE == LEVEL_RING_BYTES && (D & (D - 1)) == 0, "ring size");
+    const u32 mine = ring + (u32)lane * 16u;
+    const ulonglong2 *p[NS];
+#pragma unroll
+    for (int s = 0; s < NS; ++s) p[s] = src[s] + lane;
+    // copies chunks c and c + 32 (32 * 2 * ahead chunks past the pointers) into the stage at `to`
+    auto copy = [&](int c, int ahead, u32 to) {
+#pragma unroll
+        for (int g = 0; g < 2; ++g)
+            if (c + 32 * g < nch) {
+#pragma unroll
+                for (int s = 0; s < NS; ++s) cp16(to + (u32)(2 * s + g) * CH, p[s] + 64 * ahead + 32 * g);
+            }
+        cp_commit();
+    };
+    auto take = [&](int c, int g, u32 from) {
+        ulonglong2 v[NS];
+#pragma unroll
+        for (int s = 0; s < NS; ++s) v[s] = lds16(from + (u32)(2 * s + g) * CH);
+        f(c + 32 * g, v);
+    };
+#pragma unroll
+    for (int d = 0; d < D - 1; ++d) copy(lane + 64 * d, d, mine + d * STAGE);
+    u32 at = 0;
+    int c = lane;
+#pragma unroll 1
+    for (int whole = nch >> 6; whole > 0; --whole) {
+        copy(c + 64 * (D - 1), D - 1, mine + ((at + (D - 1) * STAGE) & (LEVEL_RING_BYTES - 1)));
+        cp_wait<D - 1>();
+        take(c, 0, mine + at);
+        take(c, 1, mine + at);
+#pragma unroll
+        for (int s = 0; s < NS; ++s) p[s] += 64;
+        c += 64;
+        at = (at + STAGE) & (LEVEL_RING_BYTES - 1);
+    }
+    cp_wait<0>();
+    if (c < nch) take(c, 0, mine + at);
+    if (c + 32 < nch) take(c, 1, mine + at);
+}
+
+// What a candidate's words are made of in a sweep: & and | are one three-input majority (l, r, o) with
+// o all zeros or all ones; U in either order; the unary operators.
+enum { SW_ANDOR = 0, SW_U = 1, SW_NEG = 2, SW_X = 3, SW_F = 4, SW_G = 5 };
+template <int SW>
+__device__ __forceinline__ u64 sweep_word(u64 l, u64 r, u64 m, u64 o, bool rl) {
+    if (SW == SW_ANDOR) return (l & r) | ((l | r) & o);
+    if (SW == SW_U) return row_until(l | r, rl ? l : r);
+    return row_unary(SW == SW_NEG ? OP_NEG : SW == SW_X ? OP_X : SW == SW_F ? OP_F : OP_G, r, m & LENMASK);
+}
+// The sweep over one candidate's words after its probe: its words into a claimed row (WRITE), or
+// compared with the stored row whose fingerprint it has (returns nonzero in a lane that found a
+// difference).
+template <int SW, bool WRITE>
+__device__ __forceinline__ u32 sweep_op(const Cand &k, const ulonglong2 *meta, ulonglong2 *row, int nch, u32 ring, int lane) {
+    constexpr bool UN = SW >= SW_NEG, META = SW == SW_NEG || SW == SW_G;
+    constexpr int NS = WRITE ? 1 : 2;
+    const u64 o = k.wop == OP_OR ? ~0ull : 0ull;
+    const bool rl = k.wop == W_URL;
+    const ulonglong2 *src[NS];
+    src[0] = k.right;
+    if (!WRITE) src[NS - 1] = row;
+    u32 d = 0;
+    const u32 left = k.left;
+    stream<NS, 4 / NS>(src, nch, ring, lane, [&](int c, const ulonglong2 (&v)[NS]) {
+        const ulonglong2 l = UN ? make_ulonglong2(0, 0) : lds16(left + (u32)c * 16u);
+        const ulonglong2 m = META ? __ldcg(meta + c) : make_ulonglong2(0, 0);
+        const u64 x = sweep_word<SW>(l.x, v[0].x, m.x, o, rl), y = sweep_word<SW>(l.y, v[0].y, m.y, o, rl);
+        if (WRITE) {
+            row[c] = make_ulonglong2(x, y);
+        } else {
+            const u64 e = (x ^ v[NS - 1].x) | (y ^ v[NS - 1].y);
+            d |= hi32(e) | (u32)e;
+        }
+    });
+    return d;
+}
+template <bool WRITE>
+__device__ __noinline__ u32 sweep(Cand k, const ulonglong2 *meta, ulonglong2 *row, int nch, u32 ring, int lane) {
+    switch (k.wop) {
+    case OP_NEG: return sweep_op<SW_NEG, WRITE>(k, meta, row, nch, ring, lane);
+    case OP_X: return sweep_op<SW_X, WRITE>(k, meta, row, nch, ring, lane);
+    case OP_F: return sweep_op<SW_F, WRITE>(k, meta, row, nch, ring, lane);
+    case OP_G: return sweep_op<SW_G, WRITE>(k, meta, row, nch, ring, lane);
+    case OP_AND:
+    case OP_OR: return sweep_op<SW_ANDOR, WRITE>(k, meta, row, nch, ring, lane);
+    default: return sweep_op<SW_U, WRITE>(k, meta, row, nch, ring, lane);
+    }
+}
 // A stored row as its own candidate (letters).
 struct RowGen {
     using Pre = ulonglong2;
@@ -249,6 +355,28 @@ __device__ __forceinline__ void count_row_stats(u64 *cnt, bool stored, u32 pmiss
     }
 }
 
+// The same for one row: it holds on every positive, on no negative.  Lane 0 counts.
+__device__ __forceinline__ void count_stats(u64 *cnt, bool every_pos, bool no_neg, int lane) {
+    if (lane == 0) {
+        if (every_pos) atomicAdd(cnt + 0, 1ull);
+        if (no_neg) atomicAdd(cnt + 1, 1ull);
+    }
+}
+// The counts for a row of which each lane has just written the chunks it reads here.  One warp.
+__device__ __noinline__ void count_one_row(const InstArgs &A, int cost, const ulonglong2 *row, int lane) {
+    const int nch = A.pitch >> 1;
+    u32 pm = 0, nh = 0;
+    for (int c = lane; c < nch; c += 32) {
+        const ulonglong2 w = row[c];
+        const u32 p0 = 2 * c < A.npos ? ROW_BIT0_HI : 0u, p1 = 2 * c + 1 < A.npos ? ROW_BIT0_HI : 0u;
+        pm |= pmiss2(w.x, w.y, p0, p1);
+        nh |= nhit2(w.x, w.y, p0, p1);
+    }
+    count_stats(A.lstats + (u64)cost * LSTATS, !__any_sync(FULL, pm), !__any_sync(FULL, nh), lane);
+}
+
+// Lane t owns candidate t (t < NC).  Claims are written and
+// published before any lane waits on another warp's publication, so waits cannot cycle.
 // Lane t owns candidate t (t < NC).  Every phase that touches whole CSs (writing the
 // claimed rows, verifying fingerprint matches) is one chunk-major sweep over all the
 // candidates concerned, so their loads are in flight together.  Claims are written and
@@ -285,10 +413,10 @@ __device__ void take_over(const InstArgs &A, InstCtl *C, const Gen &g, int t, u6
     atomicOr(&C->status, ST_WAIT);
 }
 
-template <int NC, class Gen>
+template <int NC, bool WIDE, class Gen>
 __device__ __forceinline__ void resolve(const InstArgs &A, InstCtl *C, int cost, const Gen &g, u64 fp, bool active,
                                         u64 parent, u64 kh, u64 kl, u64 prio, u32 anyp, u32 anyn, int *overflowed,
-                                        int lane) {
+                                        u32 ring, int lane) {
     int state = active ? S_PROBE : S_DONE;
     const u64 tagbits = (fp >> 40) << 40;
     const u64 genbits = (u64)A.gen << 32;
@@ -350,18 +478,29 @@ __device__ __forceinline__ void resolve(const InstArgs &A, InstCtl *C, int cost,
             if (lane == leader) base = atomicAdd(&C->row_count, (u64)__popc(cm));
             base = __shfl_sync(FULL, base, leader);
             const u64 cap = (u64)A.cap_rows;
-            ulonglong2 *out[NC];
-            u32 wm = 0;  // the claims that found a row
+            if constexpr (WIDE) {
+                u64 row = base;
+#pragma unroll 1
+                for (u32 m = cm; m && row < cap; m &= m - 1u, ++row) {
+                    ulonglong2 *out = reinterpret_cast<ulonglong2 *>(A.cache + row * pitch);
+                    sweep<true>(g.cand(__ffs(m) - 1), reinterpret_cast<const ulonglong2 *>(A.wmeta), out, nch, ring, lane);
+                    if (A.lstats) count_one_row(A, cost, out, lane);
+                }
+            } else {
+                ulonglong2 *out[NC];
+                u32 wm = 0;  // the claims that found a row
 #pragma unroll
-            for (int t = 0; t < NC; ++t) {
-                const u64 row = base + __popc(cm & ((1u << t) - 1u));
-                out[t] = reinterpret_cast<ulonglong2 *>(A.cache + row * pitch);
-                if (((cm >> t) & 1u) && row < cap) wm |= 1u << t;
+                for (int t = 0; t < NC; ++t) {
+                    const u64 row = base + __popc(cm & ((1u << t) - 1u));
+                    out[t] = reinterpret_cast<ulonglong2 *>(A.cache + row * pitch);
+                    if (((cm >> t) & 1u) && row < cap) wm |= 1u << t;
+                }
+                for (int c = lane; c < nch; c += 32)
+                    g.each(c, g.pre(c), wm, [&](int t, u64 x, u64 y) { out[t][c] = make_ulonglong2(x, y); });
             }
-            for (int c = lane; c < nch; c += 32)
-                g.each(c, g.pre(c), wm, [&](int t, u64 x, u64 y) { out[t][c] = make_ulonglong2(x, y); });
             const u64 myrow = base + __popc(cm & ((1u << lane) - 1u));
-            if (A.lstats) count_row_stats(A.lstats + (u64)cost * LSTATS, state == S_CLAIM && myrow < cap, anyp, anyn, lane);
+            if (!WIDE && A.lstats)
+                count_row_stats(A.lstats + (u64)cost * LSTATS, state == S_CLAIM && myrow < cap, anyp, anyn, lane);
             if (state == S_CLAIM && myrow < cap) {
                 A.parents[myrow] = parent;
                 if (A.keys) {
@@ -404,26 +543,38 @@ __device__ __forceinline__ void resolve(const InstArgs &A, InstCtl *C, int cost,
         if (A.key_mode == KEY_EXACT) {
             const u32 vm = __ballot_sync(FULL, state == S_VERIFY);
             if (vm) {
-                u32 diffs[NC];
-                const u32 myv = (u32)vrow;
-                const ulonglong2 *vr[NC];
-#pragma unroll
-                for (int t = 0; t < NC; ++t) diffs[t] = 0;
-#pragma unroll
-                for (int t = 0; t < NC; ++t)
-                    vr[t] = reinterpret_cast<const ulonglong2 *>(A.cache + (u64)__shfl_sync(FULL, myv, t) * pitch);
+                u32 anydiff = 0;
+                if constexpr (WIDE) {
 #pragma unroll 1
-                for (int c = lane; c < nch; c += 32) {
-                    g.each(c, g.pre(c), vm, [&](int t, u64 x, u64 y) {
-                        const ulonglong2 b = __ldcg(vr[t] + c);
-                        const u64 d = (x ^ b.x) | (y ^ b.y);
-                        diffs[t] |= hi32(d) | (u32)d;
-                    });
-                }
-                u32 diff = 0;
+                    for (u32 m = vm; m; m &= m - 1u) {
+                        const int t = __ffs(m) - 1;
+                        u64 *stored = A.cache + (u64)__shfl_sync(FULL, (u32)vrow, t) * pitch;
+                        const u32 d = sweep<false>(g.cand(t), reinterpret_cast<const ulonglong2 *>(A.wmeta),
+                                                   reinterpret_cast<ulonglong2 *>(stored), nch, ring, lane);
+                        if (__any_sync(FULL, d)) anydiff |= 1u << t;
+                    }
+                } else {
+                    u32 diffs[NC];
+                    const u32 myv = (u32)vrow;
+                    const ulonglong2 *vr[NC];
 #pragma unroll
-                for (int t = 0; t < NC; ++t) diff |= diffs[t] ? 1u << t : 0u;
-                const u32 anydiff = __reduce_or_sync(FULL, diff);
+                    for (int t = 0; t < NC; ++t) diffs[t] = 0;
+#pragma unroll
+                    for (int t = 0; t < NC; ++t)
+                        vr[t] = reinterpret_cast<const ulonglong2 *>(A.cache + (u64)__shfl_sync(FULL, myv, t) * pitch);
+#pragma unroll 1
+                    for (int c = lane; c < nch; c += 32) {
+                        g.each(c, g.pre(c), vm, [&](int t, u64 x, u64 y) {
+                            const ulonglong2 b = __ldcg(vr[t] + c);
+                            const u64 d = (x ^ b.x) | (y ^ b.y);
+                            diffs[t] |= hi32(d) | (u32)d;
+                        });
+                    }
+                    u32 diff = 0;
+#pragma unroll
+                    for (int t = 0; t < NC; ++t) diff |= diffs[t] ? 1u << t : 0u;
+                    anydiff = __reduce_or_sync(FULL, diff);
+                }
                 if (state == S_VERIFY) {
                     if ((anydiff >> lane) & 1u) {
                         state = S_PROBE;
@@ -449,17 +600,17 @@ __device__ __forceinline__ void resolve(const InstArgs &A, InstCtl *C, int cost,
 // Fingerprints, acceptance, the find record, uniqueness for NC candidates of one warp.
 // fails[t]: this lane's words of candidate t at position 0 (fails2); bp, bn: the row statistics'
 // bits (pmiss2, nhit2), kept only when the learn counts them.  pos_of(t): block position of candidate t (the find record is per block).
-template <int NC, class Gen, class ParentOf, class PosOf, class TidOf>
+template <int NC, bool WIDE, class Gen, class ParentOf, class PosOf, class TidOf>
 __device__ __forceinline__ void finish(const InstArgs &A, InstCtl *C, Slot &sl, const Gen &g, u64 (&h)[NC],
                                        u32 (&fails)[NC], u32 bp, u32 bn, u32 valid, ParentOf parent_of, PosOf pos_of,
-                                       TidOf tid_of, int lane) {
+                                       TidOf tid_of, u32 ring, int lane) {
     const u64 sum = reduce_to_lane<NC>(h, lane);
     u32 fb = 0;
 #pragma unroll
     for (int t = 0; t < NC; ++t) fb |= (fails[t] & ROW_BIT0_HI) ? 1u << t : 0u;
     const u32 acc = ~__reduce_or_sync(FULL, fb) & valid;
     u32 anyp = 0, anyn = 0;
-    if (A.lstats) {
+    if (!WIDE && A.lstats) {
         anyp = __reduce_or_sync(FULL, bp);
         anyn = __reduce_or_sync(FULL, bn);
     }
@@ -499,14 +650,14 @@ __device__ __forceinline__ void finish(const InstArgs &A, InstCtl *C, Slot &sl, 
     // once the language cache has overflowed, the level's remaining CSs are not stored and take
     // no hash slots
     const bool room = *(volatile int *)&sl.overflowed == 0;
-    resolve<NC>(A, C, cost, g, fp, room && ((valid >> lane) & 1u), myparent, kh, kl, prio, anyp, anyn, &sl.overflowed,
-                lane);
+    resolve<NC, WIDE>(A, C, cost, g, fp, room && ((valid >> lane) & 1u), myparent, kh, kl, prio, anyp, anyn,
+                      &sl.overflowed, ring, lane);
 }
 
 // ---------------------------------------------------------------- rows
 // Binary unit: right row r (at R) against nl left rows of the slot's tile (row l_first and up),
 // every operator of MODE on each pair: NL * mode_ops(MODE) candidates.  Chunks are 16 bytes (two
-// words); two are in flight per lane.  Positives are the first npos words, so acceptance needs no
+// words); two are in flight per lane, or four on wide rows (stream).  Positives are the first npos words, so acceptance needs no
 // metadata.
 //
 // The sweep is bound by integer issue (ALU and the wide multiply-add), so it is laid out to share
@@ -515,9 +666,9 @@ __device__ __forceinline__ void finish(const InstArgs &A, InstCtl *C, Slot &sl, 
 // Measured with one operator at a time against all of them on one load (whole learns, unit or
 // near-unit costs): 1000 traces to cost 8 1.35 -> 1.14 ms, 4000 traces 10.4 -> 8.9 ms, 512 small
 // instances in a batch 18.8 -> 14.2 ms.
-template <int MODE, int NL, int HK>
+template <int MODE, int NL, int HK, bool WIDE>
 __device__ __forceinline__ void binary_unit(const InstArgs &A, InstCtl *C, Slot &sl, const ulonglong2 *tile, int nl,
-                                            long long l_first, const ulonglong2 *R, long long r, int lane) {
+                                            long long l_first, const ulonglong2 *R, long long r, u32 ring, int lane) {
     constexpr int OPS = mode_ops(MODE), NC = NL * OPS;
     const int nch = A.pitch >> 1, npos = A.npos, n = A.n;
     const int rop = sl.op;
@@ -528,45 +679,54 @@ __device__ __forceinline__ void binary_unit(const InstArgs &A, InstCtl *C, Slot 
         h[t] = 0;
         fails[t] = 0;
     }
-    const bool stats = A.lstats != nullptr;
+    const bool stats = !WIDE && A.lstats != nullptr;
     u32 bp = 0, bn = 0;
-    constexpr int CH = 2;  // right-row chunks in flight per lane
     u64 k = (2ull * (u64)lane + 1ull) * WEYL;
-    for (int c0 = lane; c0 < nch; c0 += 32 * CH) {
-        ulonglong2 rvv[CH];
+    auto chunk = [&](int c, ulonglong2 rv) {
+        const u32 p0 = 2 * c < npos ? ROW_BIT0_HI : 0u, p1 = 2 * c + 1 < npos ? ROW_BIT0_HI : 0u;
+        const bool v0 = 2 * c < n, v1 = 2 * c + 1 < n;
 #pragma unroll
-        for (int u = 0; u < CH; ++u) {
-            const int c = c0 + 32 * u;
-            if (c < nch) rvv[u] = __ldcg(R + c);
-        }
-#pragma unroll
-        for (int u = 0; u < CH; ++u) {
-            const int c = c0 + 32 * u;
-            if (c < nch) {
-                const u32 p0 = 2 * c < npos ? ROW_BIT0_HI : 0u, p1 = 2 * c + 1 < npos ? ROW_BIT0_HI : 0u;
-                const bool v0 = 2 * c < n, v1 = 2 * c + 1 < n;
-#pragma unroll
-                for (int q = 0; q < NL; ++q) {
-                    if (q < nl) {
-                        pair_words<MODE>(tile[q * nch + c], rvv[u], rop, (1u << OPS) - 1u, [&](int o, u64 w0, u64 w1) {
-                            const int t = q * OPS + o;
-                            h[t] += hw<HK>(w0, k, v0) + hw<HK>(w1, k + WEYL, v1);
-                            fails[t] |= fails2(w0, w1, p0, p1);
-                            if (stats) {
-                                bp |= pmiss2(w0, w1, p0, p1) << t;
-                                bn |= nhit2(w0, w1, p0, p1) << t;
-                            }
-                        });
+        for (int q = 0; q < NL; ++q) {
+            if (q < nl) {
+                pair_words<MODE>(tile[q * nch + c], rv, rop, (1u << OPS) - 1u, [&](int o, u64 w0, u64 w1) {
+                    const int t = q * OPS + o;
+                    h[t] += hw<HK>(w0, k, v0) + hw<HK>(w1, k + WEYL, v1);
+                    fails[t] |= fails2(w0, w1, p0, p1);
+                    if (stats) {
+                        bp |= pmiss2(w0, w1, p0, p1) << t;
+                        bn |= nhit2(w0, w1, p0, p1) << t;
                     }
-                }
+                });
             }
+        }
+    };
+    if constexpr (WIDE) {
+        const ulonglong2 *const src[1] = {R};
+        stream<1, 4>(src, nch, ring, lane, [&](int c, const ulonglong2 (&v)[1]) {
+            chunk(c, v[0]);
             k += 64ull * WEYL;
+        });
+    } else {
+        constexpr int CH = 2;  // right-row chunks in flight per lane
+        for (int c0 = lane; c0 < nch; c0 += 32 * CH) {
+            ulonglong2 rvv[CH];
+#pragma unroll
+            for (int u = 0; u < CH; ++u) {
+                const int c = c0 + 32 * u;
+                if (c < nch) rvv[u] = __ldcg(R + c);
+            }
+#pragma unroll
+            for (int u = 0; u < CH; ++u) {
+                const int c = c0 + 32 * u;
+                if (c < nch) chunk(c, rvv[u]);
+                k += 64ull * WEYL;
+            }
         }
     }
     const int cnt = OPS * nl;
     const u32 valid = (1u << cnt) - 1u;
     const PairGen<MODE, NL> g{tile, R, nch, rop};
-    finish<NC>(A, C, sl, g, h, fails, bp, bn, valid,
+    finish<NC, WIDE>(A, C, sl, g, h, fails, bp, bn, valid,
                [&](int t) {
                    const u64 l = (u64)(l_first + t / OPS);
                    const int o = t % OPS;
@@ -583,7 +743,7 @@ __device__ __forceinline__ void binary_unit(const InstArgs &A, InstCtl *C, Slot 
                    const int o = t % OPS;
                    return mode_op(MODE, o, rop) == OP_U ? 2 * tid + (u64)mode_swapped(MODE, o) : tid;
                },
-               lane);
+               ring, lane);
     if (lane == 0) atomicAdd(&sl.evals, (unsigned)cnt);
 }
 
@@ -596,56 +756,66 @@ __host__ __device__ constexpr int unit_lefts(int mode) {
 }
 
 // Unary row: every operator of the slot's mask on source row s (at src; one load of each chunk).
-template <int HK>
+template <int HK, bool WIDE>
 __device__ __forceinline__ void unary_row(const InstArgs &A, InstCtl *C, Slot &sl, int mask, const ulonglong2 *src,
-                                          long long s, int lane) {
+                                          long long s, u32 ring, int lane) {
     constexpr int NC = 4;
     const int nch = A.pitch >> 1, npos = A.npos, n = A.n;
     const ulonglong2 *meta = reinterpret_cast<const ulonglong2 *>(A.wmeta);
     u64 h[NC] = {0, 0, 0, 0};
     u32 fails[NC] = {0, 0, 0, 0};
-    const bool stats = A.lstats != nullptr;
+    const bool stats = !WIDE && A.lstats != nullptr;
     u32 bp = 0, bn = 0;
-    constexpr int CH = 2;  // source-row chunks in flight per lane
     u64 k = (2ull * (u64)lane + 1ull) * WEYL;
-    for (int c0 = lane; c0 < nch; c0 += 32 * CH) {
-        ulonglong2 sv[CH], mv[CH];
+    auto chunk = [&](int c, ulonglong2 sv, ulonglong2 mv) {
+        const u32 p0 = 2 * c < npos ? ROW_BIT0_HI : 0u, p1 = 2 * c + 1 < npos ? ROW_BIT0_HI : 0u;
+        const bool v0 = 2 * c < n, v1 = 2 * c + 1 < n;
+        const u64 m0 = mv.x & LENMASK, m1 = mv.y & LENMASK;
 #pragma unroll
-        for (int u = 0; u < CH; ++u) {
-            const int c = c0 + 32 * u;
-            if (c < nch) {
-                sv[u] = __ldcg(src + c);
-                mv[u] = __ldcg(meta + c);  // a batch slot rewrites its metadata in the launch
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < CH; ++u) {
-            const int c = c0 + 32 * u;
-            if (c >= nch) continue;
-            const u32 p0 = 2 * c < npos ? ROW_BIT0_HI : 0u, p1 = 2 * c + 1 < npos ? ROW_BIT0_HI : 0u;
-            const bool v0 = 2 * c < n, v1 = 2 * c + 1 < n;
-            const u64 m0 = mv[u].x & LENMASK, m1 = mv[u].y & LENMASK;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if ((mask >> j) & 1) {
-                    const int op = unary_slot_op(j);
-                    const u64 w0 = row_unary(op, sv[u].x, m0), w1 = row_unary(op, sv[u].y, m1);
-                    h[j] += hw<HK>(w0, k, v0) + hw<HK>(w1, k + WEYL, v1);
-                    fails[j] |= fails2(w0, w1, p0, p1);
-                    if (stats) {
-                        bp |= pmiss2(w0, w1, p0, p1) << j;
-                        bn |= nhit2(w0, w1, p0, p1) << j;
-                    }
+        for (int j = 0; j < 4; ++j) {
+            if ((mask >> j) & 1) {
+                const int op = unary_slot_op(j);
+                const u64 w0 = row_unary(op, sv.x, m0), w1 = row_unary(op, sv.y, m1);
+                h[j] += hw<HK>(w0, k, v0) + hw<HK>(w1, k + WEYL, v1);
+                fails[j] |= fails2(w0, w1, p0, p1);
+                if (stats) {
+                    bp |= pmiss2(w0, w1, p0, p1) << j;
+                    bn |= nhit2(w0, w1, p0, p1) << j;
                 }
             }
+        }
+    };
+    if constexpr (WIDE) {
+        const ulonglong2 *const rows[2] = {src, meta};
+        stream<2, 2>(rows, nch, ring, lane, [&](int c, const ulonglong2 (&v)[2]) {
+            chunk(c, v[0], v[1]);
             k += 64ull * WEYL;
+        });
+    } else {
+        constexpr int CH = 2;  // source-row chunks in flight per lane
+        for (int c0 = lane; c0 < nch; c0 += 32 * CH) {
+            ulonglong2 sv[CH], mv[CH];
+#pragma unroll
+            for (int u = 0; u < CH; ++u) {
+                const int c = c0 + 32 * u;
+                if (c < nch) {
+                    sv[u] = __ldcg(src + c);
+                    mv[u] = __ldcg(meta + c);  // a batch slot rewrites its metadata in the launch
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < CH; ++u) {
+                const int c = c0 + 32 * u;
+                if (c < nch) chunk(c, sv[u], mv[u]);
+                k += 64ull * WEYL;
+            }
         }
     }
     const u32 valid = (u32)(mask & 15);
     const UnGen g{src, meta};
-    finish<NC>(A, C, sl, g, h, fails, bp, bn, valid,
+    finish<NC, WIDE>(A, C, sl, g, h, fails, bp, bn, valid,
                [&](int t) { return pack_parent(unary_slot_op(t & 3), (u64)s, 0); },
-               [&](int t) { return sl.upos[t & 3]; }, [&](int) -> u64 { return (u64)(s - sl.e_r0); }, lane);
+               [&](int t) { return sl.upos[t & 3]; }, [&](int) -> u64 { return (u64)(s - sl.e_r0); }, ring, lane);
     if (lane == 0) atomicAdd(&sl.evals, (unsigned)__popc(valid));
 }
 
@@ -1356,18 +1526,20 @@ __device__ __noinline__ void next_instance(BatchDev &B, int s, bool finishing, i
         u64 j = 0;
         if (lane == 0) j = atomicAdd(&B.next, 1ull);
         j = __shfl_sync(FULL, j, 0);
-        if (j >= (u64)B.count) {
+        if (j >= (u64)B.pending) {
             if (finishing && lane == 0) atomicSub(&B.live, 1);
             __syncwarp();
             return;
         }
-        if (setup_instance<HK>(B, s, (int)j, lane)) {
+        if (setup_instance<HK>(B, s, B.order ? __ldcg(B.order + j) : (int)j, lane)) {
             if (!finishing && lane == 0) atomicAdd(&B.live, 1);
             __syncwarp();
             return;
         }
     }
 }
+
+#include "local.cuh"
 
 // ---------------------------------------------------------------- the level kernel
 __device__ __forceinline__ Slot *slot_at(unsigned char *smem, int s) { return reinterpret_cast<Slot *>(smem) + s; }
@@ -1431,7 +1603,7 @@ __device__ __forceinline__ bool launch_done(const Launch &L, int lane) {
     if (L.batch) {
         bool d = true;
         if (lane == 0)
-            d = ld_volatile(&L.batch->next) >= (u64)L.batch->count && *(volatile int *)&L.batch->live == 0;
+            d = ld_volatile(&L.batch->next) >= (u64)L.batch->pending && *(volatile int *)&L.batch->live == 0;
         return __shfl_sync(FULL, d, 0);
     }
     bool all_done = true;
@@ -1683,7 +1855,8 @@ __device__ void producer(const Launch &L, unsigned char *smem, u64 *tiles, int l
 // slot is released) is the caller's.
 enum { SLOT_NEXT = 0, SLOT_CLOSE = 1 };
 template <int TL, int HK>
-__device__ __forceinline__ int take_rows(Slot &sl, int kind, const ulonglong2 *tile, int lane) {
+__device__ __forceinline__ int take_rows(Slot &sl, int kind, const ulonglong2 *tile, u32 ring, int lane) {
+    constexpr bool WIDE = TL == 2;
     const InstArgs &A = sl.args;
     InstCtl *C = A.ctl;
     int out = SLOT_NEXT;
@@ -1701,20 +1874,20 @@ __device__ __forceinline__ int take_rows(Slot &sl, int kind, const ulonglong2 *t
             if (kind == ENT_UNARY) {
                 int mask = sl.op;
                 for (int q = 0; q < part && split > 1; ++q) mask &= mask - 1;  // the part-th operator
-                unary_row<HK>(A, C, sl, split > 1 ? (mask & -mask) : mask, rp, r, lane);
+                unary_row<HK, WIDE>(A, C, sl, split > 1 ? (mask & -mask) : mask, rp, r, ring, lane);
             } else {
                 const int nch = A.pitch >> 1, first = part * sl.lefts;
                 const ulonglong2 *t0 = tile + (u64)first * (u64)nch;
                 const int nl = min(sl.lefts, sl.nl - first);
                 const long long lf = sl.l_first + first;
                 if (kind == ENT_ALL)
-                    binary_unit<M_ALL, unit_lefts<TL>(M_ALL), HK>(A, C, sl, t0, nl, lf, rp, r, lane);
+                    binary_unit<M_ALL, unit_lefts<TL>(M_ALL), HK, WIDE>(A, C, sl, t0, nl, lf, rp, r, ring, lane);
                 else if (kind == ENT_AO)
-                    binary_unit<M_AO, unit_lefts<TL>(M_AO), HK>(A, C, sl, t0, nl, lf, rp, r, lane);
+                    binary_unit<M_AO, unit_lefts<TL>(M_AO), HK, WIDE>(A, C, sl, t0, nl, lf, rp, r, ring, lane);
                 else if (kind == ENT_U)
-                    binary_unit<M_U, unit_lefts<TL>(M_U), HK>(A, C, sl, t0, nl, lf, rp, r, lane);
+                    binary_unit<M_U, unit_lefts<TL>(M_U), HK, WIDE>(A, C, sl, t0, nl, lf, rp, r, ring, lane);
                 else
-                    binary_unit<M_ONE, unit_lefts<TL>(M_ONE), HK>(A, C, sl, t0, nl, lf, rp, r, lane);
+                    binary_unit<M_ONE, unit_lefts<TL>(M_ONE), HK, WIDE>(A, C, sl, t0, nl, lf, rp, r, ring, lane);
             }
         }
         unsigned d = 0;
@@ -1739,7 +1912,7 @@ __device__ __forceinline__ int take_rows(Slot &sl, int kind, const ulonglong2 *t
 // A consumer warp: takes the rows of the slots in order until the producer's end slot; the
 // warp that finishes a level's last item closes the level (and plans the next one).
 template <int TL, int HK>
-__device__ void consumer(const Launch &L, unsigned char *smem, const u64 *tiles, int lane) {
+__device__ void consumer(const Launch &L, unsigned char *smem, const u64 *tiles, u32 ring, int lane) {
     const int S = L.stages;
     const long long tile_words = L.tile_bytes / 8;
     for (u64 k = 0;; ++k) {
@@ -1755,7 +1928,7 @@ __device__ void consumer(const Launch &L, unsigned char *smem, const u64 *tiles,
         const int kind = *(volatile int *)&sl.kind;
         if (kind == 0) return;
         const ulonglong2 *tile = reinterpret_cast<const ulonglong2 *>(tiles + (u64)s * tile_words);
-        const int got = take_rows<TL, HK>(sl, kind, tile, lane);
+        const int got = take_rows<TL, HK>(sl, kind, tile, ring, lane);
         int recycle = -1;  // a batch slot whose instance's search ended in this warp
         if (got == SLOT_CLOSE) {  // the slot's arguments are read before the slot is released
             const bool ended = close_level(sl.args, sl.args.ctl, L.persist != 0, lane);
@@ -1775,16 +1948,19 @@ namespace {
 __device__ __forceinline__ size_t slots_bytes(int S) { return ((size_t)S * sizeof(Slot) + 127) & ~(size_t)127; }
 
 template <int TL, int HK>
-__global__ void __launch_bounds__(LEVEL_THREADS, 1) level_kernel(const Launch *__restrict__ Lp) {
+__global__ void __launch_bounds__(level_threads(TL), 1) level_kernel(const Launch *__restrict__ Lp) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ Launch L;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // the search ended before the launch (on the small levels): nothing to do
+    if (!Lp->batch && Lp->persist && Lp->ninst == 1 && (ctl_of(*Lp, 0)->flags & CTL_DONE)) return;
+    if (Lp->batch && Lp->batch->pending == 0) return;
     if (threadIdx.x == 0) {
         L = *Lp;
         for (int s = 0; s < L.stages; ++s) {
             Slot &sl = *slot_at(smem, s);
             mbar_init(&sl.full, 1);
-            mbar_init(&sl.empty, NCONS);
+            mbar_init(&sl.empty, level_threads(TL) / 32 - 1);
         }
         fence_mbar_init();
     }
@@ -1793,7 +1969,8 @@ __global__ void __launch_bounds__(LEVEL_THREADS, 1) level_kernel(const Launch *_
     if (warp == 0)
         producer<TL>(L, smem, tiles, lane);
     else
-        consumer<TL, HK>(L, smem, tiles, lane);
+        consumer<TL, HK>(L, smem, tiles,
+                         smem_u32(tiles) + (u32)(L.stages * L.tile_bytes) + (u32)(warp - 1) * LEVEL_RING_BYTES, lane);
 }
 
 // A batch's first instances: block s sets slot s up (one warp per slot).
@@ -1920,9 +2097,15 @@ __global__ void insert_letters_kernel(const InstArgs *__restrict__ pA, int nalph
 }
 
 // Tree of the found candidate: entries (row, parents) breadth first; entry 0 is the root
-// (row ~0).  out[0] = entries written, out[1] = 1 when the buffer was too small.
-__global__ void walk_kernel(const u64 *parents, int nalpha, u64 found, u64 *out, int cap) {
+// (row ~0).  out[0] = entries written, out[1] = 1 when the buffer was too small.  The find is
+// `found`, or with a control block the one recorded there (none: no entries).
+__global__ void walk_kernel(const u64 *parents, int nalpha, u64 found, const InstCtl *ctl, u64 *out, int cap) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    if (ctl) found = ctl->found;
+    if (!found) {
+        out[0] = out[1] = 0;
+        return;
+    }
     u64 *e = out + 2;
     int count = 0, head = 0, overflow = 0;
     e[0] = ~0ull;
@@ -2043,10 +2226,10 @@ cudaError_t smem_attr(size_t smem) {
 
 template <int TL, int HK>
 cudaError_t launch_tl(const Launch &h, const Launch *d, int grid, cudaStream_t s) {
-    const size_t smem = level_kernel_smem(h.stages, h.tile_bytes);
+    const size_t smem = level_kernel_smem(h.tile, h.stages, h.tile_bytes);
     cudaError_t e = smem_attr<TL, HK>(smem);
     if (e != cudaSuccess) return e;
-    level_kernel<TL, HK><<<grid, LEVEL_THREADS, smem, s>>>(d);
+    level_kernel<TL, HK><<<grid, level_threads(TL), smem, s>>>(d);
     return cudaGetLastError();
 }
 
@@ -2054,7 +2237,7 @@ template <int TL, int HK>
 int occupancy_tl(size_t smem) {
     if (smem_attr<TL, HK>(smem) != cudaSuccess) return 0;
     int n = 0;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, level_kernel<TL, HK>, LEVEL_THREADS, smem) ==
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, level_kernel<TL, HK>, level_threads(TL), smem) ==
                    cudaSuccess
                ? n
                : 0;
@@ -2062,23 +2245,25 @@ int occupancy_tl(size_t smem) {
 
 template <int HK>
 cudaError_t launch_hk(const Launch &h, const Launch *d, int grid, cudaStream_t s) {
-    return h.tile == 2   ? launch_tl<2, HK>(h, d, grid, s)
+    return h.tile <= 2   ? launch_tl<2, HK>(h, d, grid, s)
            : h.tile == 4 ? launch_tl<4, HK>(h, d, grid, s)
                          : launch_tl<8, HK>(h, d, grid, s);
 }
 
 }  // namespace
 
-size_t level_kernel_smem(int stages, long long tile_bytes) {
-    return (((size_t)stages * sizeof(Slot) + 127) & ~(size_t)127) + (size_t)stages * (size_t)tile_bytes;
+size_t level_kernel_smem(int tile, int stages, long long tile_bytes) {
+    return (((size_t)stages * sizeof(Slot) + 127) & ~(size_t)127) + (size_t)stages * (size_t)tile_bytes +
+           (size_t)level_ring_bytes(tile);
 }
 
 cudaError_t launch_levels(const Launch &h, const Launch *d, int grid, int hk, cudaStream_t s) {
     return hk == 1 ? launch_hk<1>(h, d, grid, s) : launch_hk<0>(h, d, grid, s);
 }
 
-int level_kernel_ctas_per_sm(int hk, size_t smem) {
-    // every tile instance has the same resource use up to its registers; ask the 8-row one
+int level_kernel_ctas_per_sm(int tile, int hk, size_t smem) {
+    if (tile <= 2) return hk == 1 ? occupancy_tl<2, 1>(smem) : occupancy_tl<2, 0>(smem);
+    // the other tile instances have the same resource use up to their registers; ask the 8-row one
     return hk == 1 ? occupancy_tl<8, 1>(smem) : occupancy_tl<8, 0>(smem);
 }
 
@@ -2095,6 +2280,48 @@ cudaError_t launch_batch_start(BatchDev *d, int nslots, int hk, cudaStream_t s) 
     return cudaGetLastError();
 }
 
+cudaError_t launch_init(const InstArgs *d, const StartIn *in, int pitch, cudaStream_t s) {
+    init_kernel<<<(pitch + 127) / 128, 128, 0, s>>>(d, in);
+    return cudaGetLastError();
+}
+
+bool local_takes(int key_mode, int pitch) { return key_mode != KEY_REF && pitch <= LPITCH; }
+
+template <int HK>
+static cudaError_t launch_start_hk(const InstArgs *d, const StartIn *in, cudaStream_t s) {
+    // the shared-memory limit is a per-device attribute of the kernel: set once on each device
+    static std::atomic<unsigned long long> done{0};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev >= 64 || !((done.load() >> dev) & 1ull)) {
+        e = cudaFuncSetAttribute(start_kernel<HK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Local));
+        if (e != cudaSuccess) return e;
+        if (dev < 64) done.fetch_or(1ull << dev);
+    }
+    start_kernel<HK><<<1, LT_ONE, sizeof(Local), s>>>(d, in, LOCAL_LEVEL_WORK);
+    return cudaGetLastError();
+}
+
+template <int HK>
+static cudaError_t launch_batch_local_hk(BatchDev *d, const InstArgs *args, long long words, long long limit, int ctas,
+                                         cudaStream_t s) {
+    cudaError_t e = cudaFuncSetAttribute(batch_local_kernel<HK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Local));
+    if (e != cudaSuccess) return e;
+    batch_local_kernel<HK><<<ctas, LT_BATCH, sizeof(Local), s>>>(d, args, words, limit);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_batch_local(BatchDev *d, const InstArgs *args, long long words, long long limit, int ctas, int hk,
+                               cudaStream_t s) {
+    return hk == 1 ? launch_batch_local_hk<1>(d, args, words, limit, ctas, s)
+                   : launch_batch_local_hk<0>(d, args, words, limit, ctas, s);
+}
+
+cudaError_t launch_start(const InstArgs *d, const StartIn *in, int hk, cudaStream_t s) {
+    return hk == 1 ? launch_start_hk<1>(d, in, s) : launch_start_hk<0>(d, in, s);
+}
+
 cudaError_t launch_plan_level(const InstArgs *d, int cost, cudaStream_t s) {
     plan_only_kernel<<<1, 32, 0, s>>>(d, cost);
     return cudaGetLastError();
@@ -2109,8 +2336,8 @@ cudaError_t launch_insert_letters(const InstArgs *d, int nalpha, int hk, cudaStr
     return cudaGetLastError();
 }
 
-cudaError_t launch_walk(const u64 *parents, int nalpha, u64 found, u64 *out, int cap, cudaStream_t s) {
-    walk_kernel<<<1, 32, 0, s>>>(parents, nalpha, found, out, cap);
+cudaError_t launch_walk(const u64 *parents, int nalpha, u64 found, const InstCtl *ctl, u64 *out, int cap, cudaStream_t s) {
+    walk_kernel<<<1, 32, 0, s>>>(parents, nalpha, found, ctl, out, cap);
     return cudaGetLastError();
 }
 

@@ -227,6 +227,9 @@ struct BatchDev {
     u64 *t0;                   // per slot: globaltimer at its set-up
     long long cache_words;     // per slot: language-cache words
     long long max_rows;        // per slot: rows of parents (and keys)
+    int *order;                // the pending instances (null: 0 .. pending - 1)
+    unsigned long long next_local;  // next instance batch_local_kernel takes
+    int pending;               // instances for the slots
     int count;                 // instances
     int nslots;
     int max_pitch;
@@ -278,11 +281,18 @@ __host__ __device__ inline BlockInfo block_info(int op, int c, int lcost, long l
     return bi;
 }
 
-// Threads per CTA of the level kernel (one producer warp and the consumer warps).
+// Threads per CTA of the level kernel (one producer warp and the consumer warps) for a left tile.
+// Wide rows (tiles of one or two rows: more than about 2,100 traces) stream through shared-memory
+// rings and take more registers; narrower rows do better with more warps, each loading into registers
+// (levels of 97 thousand candidates: 264 traces 130 us, with rings 184; 500 traces 163 and 227; 1000
+// traces even; 3000 traces, 64-bit fingerprints, whole learn 1.92 and 1.65 ms; 4000 traces 8.9 and 7.8).
 constexpr int LEVEL_THREADS = 1024;
-constexpr int LEVEL_CONSUMERS = LEVEL_THREADS / 32 - 1;
+constexpr int LEVEL_THREADS_WIDE = 640;
+constexpr int LEVEL_RING_BYTES = 4096;  // shared memory of a consumer warp's load ring (wide rows)
+__host__ __device__ constexpr int level_threads(int tile) { return tile <= 2 ? LEVEL_THREADS_WIDE : LEVEL_THREADS; }
+constexpr int level_ring_bytes(int tile) { return tile <= 2 ? (LEVEL_THREADS_WIDE / 32 - 1) * LEVEL_RING_BYTES : 0; }
 // Shared memory of one CTA of the level kernel for `stages` slots of tile_bytes each.
-size_t level_kernel_smem(int stages, long long tile_bytes);
+size_t level_kernel_smem(int tile, int stages, long long tile_bytes);
 
 // Launch wrappers (learn.cu).  The kernels read their arguments from device memory, so a
 // launch (or a captured graph) stays valid while the arguments change between learns.
@@ -291,12 +301,37 @@ cudaError_t launch_first_plan(const InstArgs *d, int ninst, int open, cudaStream
 // A batch's first instances: each slot takes pending instances until one needs levels.
 cudaError_t launch_batch_start(BatchDev *d, int nslots, int hash_kind, cudaStream_t s);
 cudaError_t launch_insert_letters(const InstArgs *d, int nalpha, int hash_kind, cudaStream_t s);
-cudaError_t launch_walk(const u64 *parents, int nalpha, u64 found, u64 *out, int cap, cudaStream_t s);
+cudaError_t launch_walk(const u64 *parents, int nalpha, u64 found, const InstCtl *ctl, u64 *out, int cap, cudaStream_t s);
+// An instance's traces as the set-up kernels read them.
+struct StartIn {
+    const void *steps;       // step masks, shifted down to the lowest letter: `width` bytes each (1, 2 or 4)
+    const int *offs;         // n + 1, relative to steps
+    int width;
+    char bit[28];            // each letter's bit in the masks
+};
+// Set-up of an instance (letters, word metadata, level arrays, control block) from its traces.
+cudaError_t launch_init(const InstArgs *d, const StartIn *in, int pitch, cudaStream_t s);
+// Set-up, the small levels on one CTA, and the plan of the first larger level (csrc/local.cuh); only
+// where local_takes says so.
+bool local_takes(int key_mode, int pitch);
+cudaError_t launch_start(const InstArgs *d, const StartIn *in, int hash_kind, cudaStream_t s);
+// The instances of a batch that end on small levels, one per CTA (args: per CTA, `words` words of rows each).
+constexpr int LOCAL_BATCH_FACTOR = 12;  // how much larger levels a CTA takes when every SM has instances
+constexpr int LOCAL_ROWS = 5120;  // rows a CTA takes an instance to
+constexpr int LOCAL_COSTS = 65;   // level-array entries it uses
+cudaError_t launch_batch_local(BatchDev *d, const InstArgs *args, long long words, long long limit, int ctas, int hash_kind,
+                               cudaStream_t s);
+// Units x (32-chunk steps + 1) of a level that one CTA takes.  One SM does a tiny level in 7 us where the
+// queue takes 23 to 50, and falls behind as soon as there is work for more: at 40 traces 121 units take
+// 25 us here and 22 there, 183 take 24 and 33; at 132 traces 121 units (363 in this measure were they
+// one warp wide) 75 and 29; at 1000 traces 21 units 48 and 50, 73 units 114 and 43.  Bounds of 300, 600,
+// 1200 and 3000 give 24 small sub-problems 2.80, 2.82, 3.01 and 3.09 ms.
+constexpr long long LOCAL_LEVEL_WORK = 400;
 // Plans level `cost` of the instance from its level starts (the levels below must be complete) and
 // publishes the plan closed: the host opens it (host-driven levels, block labels).
 cudaError_t launch_plan_level(const InstArgs *d, int cost, cudaStream_t s);
 cudaError_t launch_scorer_pack(const float *params, MlpDev *out, cudaStream_t s);
-int level_kernel_ctas_per_sm(int hash_kind, size_t smem);
+int level_kernel_ctas_per_sm(int tile, int hash_kind, size_t smem);
 // prog: (op, arg) pairs in postfix, op OP_ATOM with arg = letter index; stack: depth x n words.
 cudaError_t launch_eval_formula(const int *prog, int len, const u64 *atoms, const u64 *lenmask, int n, u64 *stack,
                                 u64 *out, cudaStream_t s);

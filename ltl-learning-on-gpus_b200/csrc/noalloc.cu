@@ -235,7 +235,7 @@ extern "C" LTLG_API int ltlg_learn_noalloc(const ltlg_traces *t, const ltlg_opti
     const int hk = opt->key_mode == LTLG_KEY_HASH64 ? 1 : 0;
     int num_sms = 0;
     cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
-    const int per_sm = level_kernel_ctas_per_sm(hk, level_kernel_smem(stages, tile_bytes));
+    const int per_sm = level_kernel_ctas_per_sm(tile, hk, level_kernel_smem(tile, stages, tile_bytes));
     const int grid = (num_sms > 0 ? num_sms : 1) * (per_sm > 0 ? per_sm : 1);
 
     // Inputs and zeroed state (default stream, synchronous copies from stack arrays).
@@ -350,7 +350,7 @@ extern "C" LTLG_API int ltlg_learn_noalloc(const ltlg_traces *t, const ltlg_opti
     }
     const u64 p = hc.found & ~(1ull << 63);
 
-    if ((err = launch_walk(parents, nalpha, hc.found, walk, WALK_CAP, 0)) != cudaSuccess) return LTLG_CUDA_ERROR;
+    if ((err = launch_walk(parents, nalpha, hc.found, nullptr, walk, WALK_CAP, 0)) != cudaSuccess) return LTLG_CUDA_ERROR;
     static_assert(WALK_CAP <= 1024, "walk entries live on the stack");
     u64 ent[2 + 2 * WALK_CAP];
     if ((err = cudaMemcpy(ent, walk, sizeof(ent), cudaMemcpyDeviceToHost)) != cudaSuccess) return LTLG_CUDA_ERROR;

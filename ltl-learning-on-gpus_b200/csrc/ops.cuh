@@ -154,6 +154,21 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, u32 bytes, 
 __device__ __forceinline__ void prefetch_l2(const void *src, u32 bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
+// 16 bytes global -> shared by this thread, through L2; a thread reads back its own copies after
+// its wait (cp_wait<N>: at most N of its groups still in flight).
+__device__ __forceinline__ void cp16(u32 dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ ulonglong2 lds16(u32 a) {
+    ulonglong2 v;
+    asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(a) : "memory");
+    return v;
+}
 __device__ __forceinline__ bool mbar_try_wait(u64 *bar, u32 parity) {
     u32 ok;
     asm volatile(
