@@ -332,9 +332,6 @@ constexpr long long LOCAL_LEVEL_WORK = 400;
 cudaError_t launch_plan_level(const InstArgs *d, int cost, cudaStream_t s);
 cudaError_t launch_scorer_pack(const float *params, MlpDev *out, cudaStream_t s);
 int level_kernel_ctas_per_sm(int tile, int hash_kind, size_t smem);
-// prog: (op, arg) pairs in postfix, op OP_ATOM with arg = letter index; stack: depth x n words.
-cudaError_t launch_eval_formula(const int *prog, int len, const u64 *atoms, const u64 *lenmask, int n, u64 *stack,
-                                u64 *out, cudaStream_t s);
 cudaError_t launch_apply_op(int op, const u64 *a, const u64 *b, const u64 *wmeta, int n, int pitch, int count,
                             u64 *out, u64 *out2, u64 *fp, cudaStream_t s);
 
