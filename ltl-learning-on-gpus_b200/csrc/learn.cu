@@ -1066,8 +1066,8 @@ __device__ void plan_level(const InstArgs &A, InstCtl *C, int c, int lane) {
     __syncwarp();
 }
 
-// Learned order (PLAN_LEARNED): every block of the plan is scored by the scorer, one block
-// at a time on this warp (lane l computes hidden units l and l + 32).  A fused unary entry's
+// Learned order (PLAN_LEARNED): every block of the plan is scored by the scorer, each lane making one
+// block's features and the warp scoring SCORE_N of them at a time.  A fused unary entry's
 // chance is that any of its operators' blocks accepts, 1 - prod(1 - p).  Entries are sorted by
 // chance / sqrt(candidates), highest first, ties in the reference's order, and their item
 // starts are laid out again in the new order.  Plans whose items all start at once
@@ -1078,38 +1078,49 @@ __device__ void score_plan(const InstArgs &A, InstCtl *C, int lane) {
     const MlpDev &M = *reinterpret_cast<const MlpDev *>(A.model);
     const int c = __ldcg(&C->plan.cost), nblocks = __ldcg(&C->plan.nblocks);
     const long long level_cands = (long long)__ldcg(&C->plan.cand);
-    for (int e = 0; e < ne; ++e) {
-        const Entry *E = A.entries + e;
-        const int kind = __ldcg(&E->kind), opmask = __ldcg(&E->opmask), lcost = __ldcg(&E->lcost);
-        const long long l0 = __ldcg(&E->l0), l1 = __ldcg(&E->l1), r0 = __ldcg(&E->r0), r1 = __ldcg(&E->r1);
-        const long long cand = (long long)__ldcg(&E->cand);
-        float miss = 1.0f;
-        for (int j = 0; j < 4; ++j) {
-            int op, position;
-            long long lrows, rrows, bc;
-            if (kind == ENT_UNARY) {
-                if (!((opmask >> j) & 1)) continue;
-                op = unary_slot_op(j);
-                position = __ldcg(&E->upos[j]);
-                lrows = r1 - r0;
-                rrows = 1;
-                bc = r1 - r0;
-            } else {
-                if (j) break;
-                op = __ldcg(&E->op);
-                position = __ldcg(&E->pos);
-                lrows = l1 - l0;
-                rrows = r1 - r0;
-                bc = cand;
+    for (int base = 0; base < 4 * ne; base += 32) {
+        // lane: operator slot j of entry e (a binary entry is slot 0)
+        const int e = (base + lane) >> 2, j = lane & 3;
+        float f[ORDER_NF];
+        bool block = false;
+        long long cand = 1;
+        if (e < ne) {
+            const Entry *E = A.entries + e;
+            const int kind = __ldcg(&E->kind), opmask = __ldcg(&E->opmask), lcost = __ldcg(&E->lcost);
+            const long long l0 = __ldcg(&E->l0), l1 = __ldcg(&E->l1), r0 = __ldcg(&E->r0), r1 = __ldcg(&E->r1);
+            const bool un = kind == ENT_UNARY;
+            cand = (long long)__ldcg(&E->cand);
+            block = un ? ((opmask >> j) & 1) != 0 : j == 0;
+            if (block) {
+                const int op = un ? unary_slot_op(j) : __ldcg(&E->op), position = un ? __ldcg(&E->upos[j]) : __ldcg(&E->pos);
+                const BlockInfo bi = block_info(op, c, lcost, un ? r1 - r0 : l1 - l0, un ? 1 : r1 - r0, un ? r1 - r0 : cand,
+                                                position, A.cf, nblocks, level_cands, A.lstats, A.max_cost, A.npos, A.n,
+                                                A.nalpha);
+                block_features(bi, f);
             }
-            const BlockInfo bi = block_info(op, c, lcost, lrows, rrows, bc, position, A.cf, nblocks, level_cands,
-                                            A.lstats, A.max_cost, A.npos, A.n, A.nalpha);
-            float f[ORDER_NF];
-            block_features(bi, f);
-            const float z = mlp_score_warp(M, f, lane);
-            miss *= 1.0f / (1.0f + expf(z));  // 1 - sigmoid(z)
         }
-        if (lane == 0) __stcg(&A.entries[e].score, (1.0f - miss) / sqrtf((float)(cand > 0 ? cand : 1)));
+        if (!block)
+            for (int i = 0; i < ORDER_NF; ++i) f[i] = 0.0f;
+        __syncwarp();
+        float miss = 1.0f;  // 1 - sigmoid of this lane's block
+        for (u32 m = __ballot_sync(FULL, block); m;) {
+            int src[SCORE_N];
+            float z[SCORE_N];
+#pragma unroll
+            for (int q = 0; q < SCORE_N; ++q) {
+                src[q] = m ? __ffs(m) - 1 : 0;
+                m &= m - 1u;
+                if (q && src[q] == 0) src[q] = src[0];
+            }
+            mlp_score_warp(M, f, src, lane, z);
+#pragma unroll
+            for (int q = 0; q < SCORE_N; ++q)
+                if (lane == src[q]) miss = 1.0f / (1.0f + expf(z[q]));
+        }
+        const float m1 = __shfl_down_sync(FULL, miss, 1), m2 = __shfl_down_sync(FULL, miss, 2),
+                    m3 = __shfl_down_sync(FULL, miss, 3);
+        miss = miss * m1 * m2 * m3;  // lane 4e: the entry's blocks, in slot order
+        if (j == 0 && e < ne) __stcg(&A.entries[e].score, (1.0f - miss) / sqrtf((float)(cand > 0 ? cand : 1)));
     }
     __syncwarp();
     __threadfence_block();

@@ -27,10 +27,13 @@ constexpr int MLP_W3 = MLP_B2 + ORDER_H;             // [H]
 constexpr int MLP_B3 = MLP_W3 + ORDER_H;             // [1]
 constexpr int MLP_PARAMS = MLP_B3 + 1;
 
-// The scorer on the device: BF16 weights, FP32 biases.
+// The scorer on the device: BF16 weights, FP32 biases.  The hidden layers' weights are kept both ways:
+// [out][in], and [in][out] for threads that each compute one unit.
 struct MlpDev {
     __nv_bfloat16 w1[ORDER_H * ORDER_NF];
     __nv_bfloat16 w2[ORDER_H * ORDER_H];
+    __nv_bfloat16 w1t[ORDER_NF * ORDER_H];
+    __nv_bfloat16 w2t[ORDER_H * ORDER_H];
     __nv_bfloat16 w3[ORDER_H];
     float b1[ORDER_H];
     float b2[ORDER_H];

@@ -103,3 +103,17 @@ def test_evaluate_depth(depth):
         a = atoms[k % 2]
         v = ((a & v, a | v, gen._until(a, v))[k % 3]) if k % 5 else gen._until(atoms[1] >> np.uint64(1), v)
     assert np.array_equal(cs, v & mask) and np.array_equal(holds, (v & np.uint64(1)).astype(bool))
+
+
+@pytest.mark.parametrize("count", [1, 15, 16, 17, 4735, 4737, 9600])
+def test_scorer_gradient_sizes(count):
+    """Groups of 16 records, the last ragged, and more groups than CTAs (296): the oracle's gradient,
+    within the bounds the scorer's other tests use (BF16 operands; relative L2 1e-2, loss 1e-4)."""
+    import scorer_oracle as S
+    rng = np.random.default_rng(count)
+    x = rng.random((count, api.SCORER_FEATURES), dtype=np.float32)
+    y = (rng.random(count) < 0.3).astype(np.float32)
+    p = (rng.standard_normal(api.SCORER_PARAMS) * 0.2).astype(np.float32)
+    g, loss = api.scorer_grad(p, x, y, pos_weight=2.0)
+    wg, wl = S.grad(p, x, y, 2.0)
+    assert np.linalg.norm(g - wg) <= 1e-2 * np.linalg.norm(wg) and abs(loss - wl) <= 1e-4 * max(1.0, abs(wl))
