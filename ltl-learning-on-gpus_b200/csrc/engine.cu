@@ -410,19 +410,22 @@ cudaError_t wait_levels(ltlg_engine *e, double t0, double time_limit_s, LoopOut 
     return cudaSuccess;
 }
 
-// Runs the level kernel once over the open window of a host-driven level and waits for it.
-cudaError_t run_levels(ltlg_engine *e, int grid, double t0, LoopOut &o) {
+// Windows of a host-driven level: begin_windows, then for each window its opening and a launch, all in
+// stream order, then end_windows waits for them (a wait after each made 25 us of a small block's 45).
+cudaError_t begin_windows(ltlg_engine *e) {
     Launch *hl = (Launch *)((char *)e->h_up.p + Up::LAUNCH);
     fill_launch(e, *hl, false);
-    cudaStream_t st = e->stream;
-    cudaError_t err = cudaMemcpyAsync(e->launch(), hl, sizeof(Launch), cudaMemcpyHostToDevice, st);
-    if (err != cudaSuccess) return err;
-    cudaEventRecord(e->ev_a, st);
-    err = launch_levels(*hl, e->launch(), grid, e->hk, st);
-    if (err != cudaSuccess) return err;
-    cudaEventRecord(e->ev_b, st);
+    cudaError_t err = cudaMemcpyAsync(e->launch(), hl, sizeof(Launch), cudaMemcpyHostToDevice, e->stream);
+    return err == cudaSuccess ? cudaEventRecord(e->ev_a, e->stream) : err;
+}
+cudaError_t run_window(ltlg_engine *e, long long items, LoopOut &o) {
     ++o.launches;
-    return wait_levels(e, t0, 0.0, o);
+    const int grid = (int)std::max<long long>(1, std::min<long long>(items, e->grid));
+    return launch_levels(*(const Launch *)((char *)e->h_up.p + Up::LAUNCH), e->launch(), grid, e->hk, e->stream);
+}
+cudaError_t end_windows(ltlg_engine *e, double t0, LoopOut &o) {
+    const cudaError_t err = cudaEventRecord(e->ev_b, e->stream);
+    return err == cudaSuccess ? wait_levels(e, t0, 0.0, o) : err;
 }
 
 cudaError_t read_ctl(ltlg_engine *e, InstCtl *hc) {
@@ -468,8 +471,7 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
     const int npos = t->num_pos, nneg = t->num_neg, n = npos + nneg;
     const std::string alpha = t->alphabet ? t->alphabet : "";
     const int nalpha = (int)alpha.size();
-    const bool ref_keys = opt->key_mode == LTLG_KEY_REF;
-    if (!traces_well_formed(t) || (ref_keys && (opt->rlx_unq_chk_type < 1 || opt->rlx_unq_chk_type > 3)) ||
+    if (!traces_well_formed(t) || (opt->key_mode == LTLG_KEY_REF && (opt->rlx_unq_chk_type < 1 || opt->rlx_unq_chk_type > 3)) ||
         opt->key_mode < 0 || opt->key_mode > 2 || n > e->cfg.max_traces || nalpha > 26 || opt->max_cost < 1 ||
         opt->max_cost > SHRT_MAX || (opt->order != LTLG_ORDER_PLAIN && opt->order != LTLG_ORDER_LEARNED) ||
         (opt->order == LTLG_ORDER_LEARNED && !e->has_scorer))
@@ -480,6 +482,10 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
         max_len = std::max(max_len, ln);
         len_sum += ln;
     }
+    // The reference's keys hold whole CSs of up to 126 positions in all (ltli6463.cu:57-73): there they are
+    // exact keys, and the exact path's small levels and fused entries serve them.
+    const int key_mode = opt->key_mode == LTLG_KEY_REF && len_sum <= 126 ? (int)LTLG_KEY_EXACT : opt->key_mode;
+    const bool ref_keys = key_mode == LTLG_KEY_REF;
     res->cost = c1;
     if ((opt->limit_traces && n > 64) || max_len > 63) {
         res->status = LTLG_INPUT_LIMITS;
@@ -539,7 +545,7 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
     int tile = 0, stages = 0;
     long long tile_bytes = 0;
     if (!geometry(e->cfg.left_tile, pitch, tile, stages, tile_bytes)) return fail_status(res, LTLG_BAD_ARGS);
-    const int hk = opt->key_mode == LTLG_KEY_HASH64 ? 1 : 0;
+    const int hk = key_mode == LTLG_KEY_HASH64 ? 1 : 0;
     const size_t smem = level_kernel_smem(tile, stages, tile_bytes);
     const int per_sm = level_kernel_ctas_per_sm(tile, hk, smem);
     if (per_sm < 1) return fail_status(res, LTLG_BAD_ARGS);
@@ -571,9 +577,9 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
     if (ref_keys) memset(kmeta, 0, (size_t)pitch * 4);
     int rlx_type = 0;
     if (ref_keys) {
-        rlx_type = len_sum > 126 ? opt->rlx_unq_chk_type : 0;
+        rlx_type = opt->rlx_unq_chk_type;
         long long start = 0;
-        const int stride = len_sum > 126 ? len_sum / 126 : 1;
+        const int stride = len_sum / 126;
         for (int i = 0; i < n; ++i) {
             const int ln = t->offsets[i + 1] - t->offsets[i];
             int count = ln, step = 1;
@@ -593,7 +599,7 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
     const long long cap_entries = entries_for(max_cost);
     const bool want_stats = opt->order == LTLG_ORDER_LEARNED || opt->record_levels >= 2;
     if ((err = ensure(e->parents, (size_t)cap_rows * 8)) != cudaSuccess) return fail_cuda(e, err, res);
-    if (opt->key_mode != LTLG_KEY_EXACT && (err = ensure(e->keys, (size_t)cap_rows * 16)) != cudaSuccess)
+    if (key_mode != LTLG_KEY_EXACT && (err = ensure(e->keys, (size_t)cap_rows * 16)) != cudaSuccess)
         return fail_cuda(e, err, res);
     if (ref_keys && (err = ensure(e->prio, (size_t)cap_rows * 8)) != cudaSuccess) return fail_cuda(e, err, res);
     const Down dl(ncost);
@@ -621,7 +627,7 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
     A.pitch = pitch;
     A.npos = npos;
     A.nalpha = nalpha;
-    A.key_mode = opt->key_mode == LTLG_KEY_EXACT ? KEY_EXACT : opt->key_mode == LTLG_KEY_REF ? KEY_REF : KEY_HASH64;
+    A.key_mode = key_mode == LTLG_KEY_EXACT ? KEY_EXACT : key_mode == LTLG_KEY_REF ? KEY_REF : KEY_HASH64;
     A.rlx_type = rlx_type;
     A.stop_at_found = opt->stop_at_found ? 1 : 0;
     A.find_first = learned ? 1 : 0;
@@ -645,7 +651,7 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
     A.slot_mask = e->nslots - 1;
     A.cache = (u64 *)e->cache.p;
     A.parents = (u64 *)e->parents.p;
-    A.keys = opt->key_mode != LTLG_KEY_EXACT ? (u64 *)e->keys.p : nullptr;
+    A.keys = key_mode != LTLG_KEY_EXACT ? (u64 *)e->keys.p : nullptr;
     A.prio = ref_keys ? (u64 *)e->prio.p : nullptr;
     A.slots = (u64 *)e->slots.p;
     A.wmeta = (const u64 *)e->wmeta.p;
@@ -782,19 +788,21 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
                 if ((err = cudaStreamSynchronize(st)) != cudaSuccess) return fail_cuda(e, err, res);
                 for (int q = 0; q < ne; ++q) order.push_back(q);
                 std::sort(order.begin(), order.end(), [&](int a, int b) { return hent[a].pos < hent[b].pos; });
+                if ((err = begin_windows(e)) != cudaSuccess) return fail_cuda(e, err, res);
                 for (size_t q = 0; q < order.size(); ++q) {
                     const Entry &E = hent[order[q]];
                     cudaMemcpyAsync((u64 *)e->snaps.p + q, &dctl->row_count, 8, cudaMemcpyDeviceToDevice, st);
                     if ((err = open_window(e, seq, E.item0, E.item0 + E.items, (int)q)) != cudaSuccess)
                         return fail_cuda(e, err, res);
-                    const int grid = (int)std::max<long long>(1, std::min<long long>(E.items, e->grid));
-                    if ((err = run_levels(e, grid, t0, o)) != cudaSuccess) return fail_cuda(e, err, res);
+                    if ((err = run_window(e, E.items, o)) != cudaSuccess) return fail_cuda(e, err, res);
                 }
+                if ((err = end_windows(e, t0, o)) != cudaSuccess) return fail_cuda(e, err, res);
                 cudaMemcpyAsync(e->h_snaps.p, e->snaps.p, order.size() * 8, cudaMemcpyDeviceToHost, st);
             } else {
                 if ((err = open_window(e, seq, 0, hc->plan.items, 0)) != cudaSuccess) return fail_cuda(e, err, res);
-                const int grid = (int)std::max<long long>(1, std::min<long long>(hc->plan.items, e->grid));
-                if ((err = run_levels(e, grid, t0, o)) != cudaSuccess) return fail_cuda(e, err, res);
+                if ((err = begin_windows(e)) != cudaSuccess || (err = run_window(e, hc->plan.items, o)) != cudaSuccess ||
+                    (err = end_windows(e, t0, o)) != cudaSuccess)
+                    return fail_cuda(e, err, res);
             }
             if ((err = read_ctl(e, hc)) != cudaSuccess) return fail_cuda(e, err, res);
             if (per_block) {
@@ -1048,14 +1056,15 @@ LTLG_API int ltlg_engine_label_blocks(ltlg_engine *e, const ltlg_traces *t, cons
     LoopOut o;
     InstCtl *dctl = e->ctl();
     static const u64 nofind = NO_FIND;
+    if ((err = begin_windows(e)) != cudaSuccess) return fail_cuda(e, err, nullptr);
     for (int q = 0; q < ne; ++q) {
         const Entry &E = hent[q];
         cudaMemcpyAsync(&dctl->found_key, &nofind, 8, cudaMemcpyHostToDevice, st);
         if ((err = open_window(e, hc->seq, E.item0, E.item0 + E.items, q)) != cudaSuccess)
             return fail_cuda(e, err, nullptr);
-        const int grid = (int)std::max<long long>(1, std::min<long long>(E.items, e->grid));
-        if ((err = run_levels(e, grid, now_s(), o)) != cudaSuccess) return fail_cuda(e, err, nullptr);
+        if ((err = run_window(e, E.items, o)) != cudaSuccess) return fail_cuda(e, err, nullptr);
     }
+    if ((err = end_windows(e, now_s(), o)) != cudaSuccess) return fail_cuda(e, err, nullptr);
     cudaMemcpyAsync(e->h_fpar.p, e->fpar.p, (size_t)nbl * 8, cudaMemcpyDeviceToHost, st);
     if ((err = cudaStreamSynchronize(st)) != cudaSuccess) return fail_cuda(e, err, nullptr);
     const u64 *won = (const u64 *)e->h_fpar.p;
