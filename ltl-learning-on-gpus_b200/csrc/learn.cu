@@ -1405,6 +1405,38 @@ __device__ void finish_instance(BatchDev &B, int s, int lane) {
     __syncwarp();
 }
 
+// Letter rows and word metadata (into A.cache, A.wmeta and `meta`) from an instance's step masks, by any
+// number of threads (tid of nt); each mask is read once for four letters.
+template <class T>
+__device__ __forceinline__ void init_traces_of(const InstArgs &A, const StartIn &in, u64 *meta, int tid, int nt) {
+    const T *steps = (const T *)in.steps;
+    const int pitch = A.pitch, n = A.n, nalpha = A.nalpha;
+    for (int i = tid; i < pitch; i += nt) {
+        int a = 0, b = 0;
+        if (i < n) {
+            a = in.offs[i];
+            b = in.offs[i + 1];
+        }
+        const u64 m = i < n ? row_lenmask(b - a) | (i < A.npos ? (1ull << 63) : 0ull) : 0ull;
+        const_cast<u64 *>(A.wmeta)[i] = m;
+        if (meta) meta[i] = m;
+        for (int j0 = 0; j0 < nalpha; j0 += 4) {  // four letters per pass over the steps
+            u64 w[4] = {0, 0, 0, 0};
+            int sh[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) sh[q] = j0 + q < nalpha ? in.bit[j0 + q] : 31;
+            for (int k = a; k < b; ++k) {
+                const u32 s = (u32)steps[k];
+                const int at = 62 - (k - a);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) w[q] |= (u64)((s >> sh[q]) & 1u) << at;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (j0 + q < nalpha) A.cache[(u64)(j0 + q) * (u64)pitch + i] = w[q];
+        }
+    }
+}
 // Sets slot s up with instance idx: letters (the first separating one may end the search here,
 // ltli6463.cu:1100-1136), word metadata, the slot's next hash-set generation, a clean control
 // block and level arrays, the letters in the hash set, then the first plan.  One warp.  Returns
@@ -1433,29 +1465,21 @@ __device__ bool setup_instance(BatchDev &B, int s, int idx, int lane) {
     }
     const u32 *steps = B.steps + in.steps0;
     const int *offs = B.offs + in.offs0;
-    // letters: rows 0 .. nalpha - 1, positives need position 0, negatives must not hold there
-    int hit = -1;
-    u64 all = 0;
-    for (int j = 0; j < nalpha; ++j) {
-        const u32 bit = 1u << (in.alpha[j] - 'a');
-        bool acc = true;
-        for (int i = lane; i < pitch; i += 32) {
-            u64 w = 0;
-            if (i < n) {
-                const int a = offs[i], b = offs[i + 1];
-                for (int k = a; k < b; ++k)
-                    if (steps[k] & bit) w |= 1ull << (62 - (k - a));
-                if (((w >> 62) != 0) != (i < npos)) acc = false;
-            }
-            __stcg(A.cache + (u64)j * pitch + i, w);
-        }
-        acc = __all_sync(FULL, acc);
-        ++all;
-        if (acc && hit < 0) {
-            hit = j;
-            if (A.stop_at_found) break;
-        }
+    // the first letter that holds first in every positive and in no negative trace
+    u32 every = ~0u, some = 0u;
+    for (int i = lane; i < n; i += 32) {
+        const int a = offs[i];
+        const u32 m = offs[i + 1] > a ? steps[a] : 0u;
+        if (i < npos)
+            every &= m;
+        else
+            some |= m;
     }
+    const u32 sep = __reduce_and_sync(FULL, every) & ~__reduce_or_sync(FULL, some);
+    int hit = -1;
+    for (int j = 0; j < nalpha && hit < 0; ++j)
+        if ((sep >> (in.alpha[j] - 'a')) & 1u) hit = j;
+    const u64 all = hit >= 0 && A.stop_at_found ? (u64)hit + 1 : (u64)nalpha;
     if (hit >= 0 && lane == 0) o.letter = hit;
     if ((hit >= 0 && A.stop_at_found) || n == 0 || nalpha == 0) {
         if (lane == 0) {
@@ -1471,15 +1495,6 @@ __device__ bool setup_instance(BatchDev &B, int s, int idx, int lane) {
         __syncwarp();
         return false;
     }
-    // word metadata: length mask | positive flag
-    for (int i = lane; i < pitch; i += 32) {
-        u64 m = 0;
-        if (i < n) {
-            const int ln = offs[i + 1] - offs[i];
-            m = row_lenmask(ln) | (i < npos ? (1ull << 63) : 0ull);
-        }
-        __stcg(const_cast<u64 *>(A.wmeta) + i, m);
-    }
     // the slot's arguments for this instance; a generation that wraps clears the set
     A.n = n;
     A.pitch = pitch;
@@ -1488,6 +1503,14 @@ __device__ bool setup_instance(BatchDev &B, int s, int idx, int lane) {
     A.rlx_type = 0;
     A.on_the_fly = 0;
     A.cap_rows = min(B.max_rows, B.cache_words / pitch);
+    {
+        StartIn si;
+        si.steps = steps;
+        si.offs = offs;
+        si.width = 4;
+        for (int q = 0; q < nalpha; ++q) si.bit[q] = (char)(in.alpha[q] - 'a');
+        init_traces_of<u32>(A, si, nullptr, lane, 32);
+    }
     if (A.gen >= 255) {
         for (u64 q = lane; q <= A.slot_mask; q += 32) __stcg(A.slots + q, 0ull);
         A.gen = 1;

@@ -477,36 +477,6 @@ __device__ void local_level(Local &S, int c, int tid) {
 
 // ---- set-up of an instance: letters and word metadata from its step masks, the level arrays and
 // the control block.  Any number of threads (tid of nt) over any number of CTAs.
-template <class T>
-__device__ __forceinline__ void init_traces_of(const InstArgs &A, const StartIn &in, u64 *meta, int tid, int nt) {
-    const T *steps = (const T *)in.steps;
-    const int pitch = A.pitch, n = A.n, nalpha = A.nalpha;
-    for (int i = tid; i < pitch; i += nt) {
-        int a = 0, b = 0;
-        if (i < n) {
-            a = in.offs[i];
-            b = in.offs[i + 1];
-        }
-        const u64 m = i < n ? row_lenmask(b - a) | (i < A.npos ? (1ull << 63) : 0ull) : 0ull;
-        const_cast<u64 *>(A.wmeta)[i] = m;
-        if (meta) meta[i] = m;
-        for (int j0 = 0; j0 < nalpha; j0 += 4) {  // four letters per pass over the steps
-            u64 w[4] = {0, 0, 0, 0};
-            int sh[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) sh[q] = j0 + q < nalpha ? in.bit[j0 + q] : 31;
-            for (int k = a; k < b; ++k) {
-                const u32 s = (u32)steps[k];
-                const int at = 62 - (k - a);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) w[q] |= (u64)((s >> sh[q]) & 1u) << at;
-            }
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (j0 + q < nalpha) A.cache[(u64)(j0 + q) * (u64)pitch + i] = w[q];
-        }
-    }
-}
 __device__ void init_traces(const InstArgs &A, const StartIn &in, u64 *meta, int tid, int nt) {
     if (in.width == 1)
         init_traces_of<unsigned char>(A, in, meta, tid, nt);
