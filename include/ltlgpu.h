@@ -90,7 +90,8 @@ typedef struct ltlg_engine_config {
     int64_t max_rows;          /* upper bound on cache rows (<= 2^30); 0 = budget only */
     int32_t max_traces;        /* largest n the engine accepts */
     int32_t block_threads;     /* kept for the layout; the level kernel runs one CTA of 1024 threads
-                                  per SM (a producer warp and 31 consumer warps) */
+                                  per SM (a producer warp and 31 consumer warps), of 640 on rows of
+                                  more than about 2,100 traces */
     int32_t left_tile;         /* left rows staged in shared memory per binary work item: 2, 4 or 8 */
     int32_t right_chunk;       /* right rows per binary work item of a large level */
     int32_t unary_rows;        /* source rows per unary work item of a large level */
