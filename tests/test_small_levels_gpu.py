@@ -72,7 +72,7 @@ def test_wide_rows(n):
 
 def test_batch_takes_small_and_large_instances():
     """Results of a batch are a single engine's, whichever kernel ended each instance's search."""
-    insts = [gen.generate(s, 2 + s % 3, 6 + 5 * (s % 7), 9 + 3 * (s % 11), 4, 30, 0.5, 3 + s % 6) for s in range(60)]
+    insts = [gen.generate(s, 2 + s % 3, 6 + 5 * (s % 7), 9 + 3 * (s % 11), 4, 30, 0.5, 3 + s % 6) for s in range(120)]
     insts += [traces(900 + k, n) for k, n in enumerate((2, 300, 1025))]
     for key in (api.KEY_EXACT, api.KEY_HASH64):
         opts = dict(max_cost=6, neg_type=1, key_mode=key)
