@@ -1148,7 +1148,7 @@ struct ltlg_batch {
     cudaStream_t stream = nullptr;
     DevBuf cache, parents, keys, hslots, wmeta, kmeta, ls, ne, lcands, entries, fpar, ctl, args;
     DevBuf bin, steps, offs, bout, cur, t0, bdev, launch, order;
-    DevBuf largs, lctl, lls, lne, llc, lpar, lmeta;  // per CTA of the small-level kernel (its rows are the slots' caches)
+    DevBuf lbuf;  // what the small-level kernel's CTAs keep (their rows are the slots' caches)
     DevBuf h_bin, h_steps, h_offs, h_bout, h_args, h_bdev, h_launch, h_largs;
     std::vector<u32> gen;          // each slot's hash-set generation after the last call
     ltlg_engine *fallback = nullptr;
@@ -1213,8 +1213,7 @@ LTLG_API void ltlg_batch_destroy(ltlg_batch *b) {
     if (b->stream) cudaStreamSynchronize(b->stream);
     for (DevBuf *x : {&b->cache, &b->parents, &b->keys, &b->hslots, &b->wmeta, &b->kmeta, &b->ls, &b->ne, &b->lcands,
                       &b->entries, &b->fpar, &b->ctl, &b->args, &b->bin, &b->steps, &b->offs, &b->bout, &b->cur,
-                      &b->t0, &b->bdev, &b->launch, &b->order, &b->largs, &b->lctl, &b->lls, &b->lne, &b->llc, &b->lpar,
-                      &b->lmeta})
+                      &b->t0, &b->bdev, &b->launch, &b->order, &b->lbuf})
         if (x->p) cudaFree(x->p);
     for (DevBuf *x : {&b->h_bin, &b->h_steps, &b->h_offs, &b->h_bout, &b->h_args, &b->h_bdev, &b->h_launch, &b->h_largs})
         if (x->p) cudaFreeHost(x->p);
@@ -1341,15 +1340,15 @@ LTLG_API int ltlg_batch_learn(ltlg_batch *b, const ltlg_traces *traces, int32_t 
         const bool local = err == cudaSuccess && min_pitch <= 1024 && nd >= b->num_sms / 2;
         const int lctas = std::min(nd, 2 * b->num_sms);
         const long long lwords = (long long)K * cache_words / std::max(lctas, 1) & ~3ll;
+        // the CTAs' arguments, then per CTA: control block, level arrays, parents, word metadata
+        auto up256 = [](size_t x) { return (x + 255) & ~(size_t)255; };
+        const size_t l_ctl = 0, l_ls = up256(sizeof(InstCtl)), l_lc = l_ls + up256(LOCAL_COSTS * 8),
+                     l_ne = l_lc + up256(LOCAL_COSTS * 8), l_par = l_ne + up256(LOCAL_COSTS * 4),
+                     l_meta = l_par + up256((size_t)LOCAL_ROWS * 8), l_args = l_meta + up256((size_t)max_pitch * 8),
+                     lbytes = l_args + up256(sizeof(InstArgs));
         if (local) {
             dev(b->order, (size_t)nd * 4);
-            dev(b->largs, (size_t)lctas * sizeof(InstArgs));
-            dev(b->lctl, (size_t)lctas * sizeof(InstCtl));
-            dev(b->lls, (size_t)lctas * LOCAL_COSTS * 8);
-            dev(b->lne, (size_t)lctas * LOCAL_COSTS * 4);
-            dev(b->llc, (size_t)lctas * LOCAL_COSTS * 8);
-            dev(b->lpar, (size_t)lctas * LOCAL_ROWS * 8);
-            dev(b->lmeta, (size_t)lctas * max_pitch * 8);
+            dev(b->lbuf, (size_t)lctas * lbytes);
             host(b->h_largs, (size_t)lctas * sizeof(InstArgs));
         }
         if (err == cudaSuccess) {
@@ -1448,26 +1447,29 @@ LTLG_API int ltlg_batch_learn(ltlg_batch *b, const ltlg_traces *traces, int32_t 
             if (err == cudaSuccess) err = cudaMemcpyAsync(b->launch.p, &L, sizeof(Launch), cudaMemcpyHostToDevice, st);
             if (local) {
                 InstArgs *la = (InstArgs *)b->h_largs.p;
+                char *lb = (char *)b->lbuf.p;
                 for (int q = 0; q < lctas; ++q) {
                     InstArgs &A = la[q];
+                    // the arguments of all CTAs come first, then each CTA's block
+                    char *mine = lb + (size_t)lctas * up256(sizeof(InstArgs)) + (size_t)q * l_args;
                     A = ha[0];
                     A.keys = nullptr;
                     A.cache = (u64 *)b->cache.p + (size_t)q * lwords;
-                    A.parents = (u64 *)b->lpar.p + (size_t)q * LOCAL_ROWS;
+                    A.parents = (u64 *)(mine + l_par);
                     A.slots = nullptr;
-                    A.wmeta = (const u64 *)b->lmeta.p + (size_t)q * max_pitch;
-                    A.ls = (long long *)b->lls.p + (size_t)q * LOCAL_COSTS;
-                    A.ne = (int *)b->lne.p + (size_t)q * LOCAL_COSTS;
-                    A.level_cands = (u64 *)b->llc.p + (size_t)q * LOCAL_COSTS;
+                    A.wmeta = (const u64 *)(mine + l_meta);
+                    A.ls = (long long *)(mine + l_ls);
+                    A.ne = (int *)(mine + l_ne);
+                    A.level_cands = (u64 *)(mine + l_lc);
                     A.entries = nullptr;
                     A.found_par = nullptr;
-                    A.ctl = (InstCtl *)b->lctl.p + q;
+                    A.ctl = (InstCtl *)(mine + l_ctl);
                 }
                 const long long limit = LOCAL_LEVEL_WORK * std::max(1, std::min(LOCAL_BATCH_FACTOR, nd / b->num_sms * LOCAL_BATCH_FACTOR / 2));
                 if (err == cudaSuccess)
-                    err = cudaMemcpyAsync(b->largs.p, la, (size_t)lctas * sizeof(InstArgs), cudaMemcpyHostToDevice, st);
+                    err = cudaMemcpyAsync(lb, la, (size_t)lctas * sizeof(InstArgs), cudaMemcpyHostToDevice, st);
                 if (err == cudaSuccess)
-                    err = launch_batch_local((BatchDev *)b->bdev.p, (const InstArgs *)b->largs.p, lwords, limit, lctas, hk, st);
+                    err = launch_batch_local((BatchDev *)b->bdev.p, (const InstArgs *)lb, lwords, limit, lctas, hk, st);
             }
             if (err == cudaSuccess) err = launch_batch_start((BatchDev *)b->bdev.p, K, hk, st);
             if (err == cudaSuccess) err = launch_levels(L, (const Launch *)b->launch.p, grid, hk, st);

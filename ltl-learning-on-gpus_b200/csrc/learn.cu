@@ -1,13 +1,14 @@
 // The level kernel of the characteristic-set (CS) enumeration for sm_100a, and the planner
 // that runs inside it.
 //
-// One CTA per SM, 32 warps.  Warp 0 is the producer: it takes work items from the instance's
+// One CTA per SM, 32 warps (20 on wide rows).  Warp 0 is the producer: it takes work items from the instance's
 // queue (a 64-bit counter tagged with the plan's sequence number), fills a ring of item slots
 // in shared memory, stages each binary item's tile of left-operand CSs with one bulk copy
 // (cp.async.bulk, no multicast, completion on the slot's mbarrier), and prefetches the item's
-// right-operand (or unary source) rows into L2 with one bulk prefetch.  Warps 1..31 are
-// consumers: they take the rows of the oldest slot one at a time, evaluate every candidate of
-// a row in registers, and run the fused epilogue per candidate: fingerprint (warp
+// right-operand (or unary source) rows into L2 with one bulk prefetch.  The other
+// warps are consumers: they take the units of the oldest slot one at a time (a right row against left
+// rows of the tile under every operator of the entry, or a source row under its unary operators),
+// evaluate the unit's candidates in registers, and run the fused epilogue per candidate: fingerprint (warp
 // reduce-scatter), acceptance (redux.sync over positive-miss / negative-hit bits of position
 // 0), the find record, exact uniqueness in an open-addressing HBM hash set (claim by CAS,
 // write the row, publish; a fingerprint match is verified word by word against the stored row,

@@ -232,8 +232,8 @@ __device__ __forceinline__ LocalCand local_cand(const Local &S, const LocalUnit 
     k.o = k.wop == OP_OR ? ~0ull : 0ull;
     return k;
 }
-// f(c, words of chunk c) over chunks c = gl, gl + P, ...: LCH chunks' operands are loaded before any of
-// their words is used (or stored), since a group's chain of loads is what a small level waits for.
+// f(c, words of chunk c) over chunks c = gl, gl + P, ...  One chunk at a time: two or four in flight spill
+// (64 registers) and made a level of 732 candidates take 34 instead of 24 us.
 constexpr int LCH = 1;
 template <class F>
 __device__ __forceinline__ void local_words(const Local &S, const LocalCand &k, int gl, int P, int nch, F f) {
@@ -297,8 +297,8 @@ __device__ __forceinline__ void local_eval(const Local &S, const LocalUnit &x, i
     }
 }
 
-// Candidate j of the round that starts at unit u0 into the set, from slot `idx`.
-__device__ __forceinline__ void local_probe(Local &S, int j, u32 idx, int p) {
+// Candidate j of the round into the set, from slot `idx` on.
+__device__ __forceinline__ void local_probe(Local &S, int j, u32 idx) {
     const u64 fp = S.sum[j];
     const bool exact = S.A.key_mode == KEY_EXACT;
     for (;; idx = (idx + 1) & (LTAB - 1)) {
@@ -388,7 +388,7 @@ __device__ void local_level(Local &S, int c, int tid) {
                 atomicMin(&S.found_key, mine[q]);
                 if (A.stop_at_found) continue;  // the last level: no dedupe
             }
-            local_probe(S, j, (u32)S.sum[j] & (LTAB - 1), 0);
+            local_probe(S, j, (u32)S.sum[j] & (LTAB - 1));
         }
         __syncthreads();
 #pragma unroll
@@ -468,7 +468,7 @@ __device__ void local_level(Local &S, int c, int tid) {
             if (nr == 0) break;
             for (int i = tid; i < nr; i += LT) {
                 const int j = S.retry[p][i];
-                local_probe(S, j, (S.idx[j] + 1u) & (LTAB - 1), p);
+                local_probe(S, j, (S.idx[j] + 1u) & (LTAB - 1));
             }
             __syncthreads();
         }
