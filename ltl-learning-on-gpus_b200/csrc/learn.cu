@@ -2049,13 +2049,15 @@ template <int TL, int HK>
 __global__ void __launch_bounds__(level_threads(TL), 1) level_kernel(const Launch *__restrict__ Lp) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ Launch L;
+    __shared__ bool nothing;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // the search ended before the launch (on the small levels): nothing to do
-    if (!Lp->batch && Lp->persist && Lp->ninst == 1 && (ctl_of(*Lp, 0)->flags & CTL_DONE)) return;
-    if (Lp->batch && Lp->batch->pending == 0) return;
     if (threadIdx.x == 0) {
         L = *Lp;
-        for (int s = 0; s < L.stages; ++s) {
+        // The search ended before the launch (on the small levels): nothing to do.  One thread reads the
+        // flag for the whole CTA: in a CTA that starts late, other CTAs set it while this one looks.
+        nothing = L.batch ? L.batch->pending == 0
+                          : L.persist && L.ninst == 1 && (*(volatile u32 *)&ctl_of(L, 0)->flags & CTL_DONE);
+        for (int s = 0; s < L.stages && !nothing; ++s) {
             Slot &sl = *slot_at(smem, s);
             mbar_init(&sl.full, 1);
             mbar_init(&sl.empty, level_threads(TL) / 32 - 1);
@@ -2063,6 +2065,7 @@ __global__ void __launch_bounds__(level_threads(TL), 1) level_kernel(const Launc
         fence_mbar_init();
     }
     __syncthreads();
+    if (nothing) return;
     u64 *tiles = reinterpret_cast<u64 *>(smem + slots_bytes(L.stages));
     if (warp == 0)
         producer<TL>(L, smem, tiles, lane);
