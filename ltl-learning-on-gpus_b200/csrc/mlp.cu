@@ -69,7 +69,9 @@ __global__ void __launch_bounds__(THREADS) grad_kernel(const MlpDev *__restrict_
                                                        const float *__restrict__ Y, const int *__restrict__ idx,
                                                        long long first, int n, float pos_weight, float inv_norm,
                                                        float *__restrict__ part, float *__restrict__ loss) {
-    __shared__ __nv_bfloat16 w1t[NF * H], w2[H * H], w2t[H * H], w3[H];
+    __shared__ __align__(16) __nv_bfloat16 w1t[NF * H], w2[H * H], w2t[H * H];  // filled 16 bytes at a time
+    __shared__ __nv_bfloat16 w3[H];
+    static_assert(__alignof__(w1t) >= 16 && __alignof__(w2) >= 16 && __alignof__(w2t) >= 16, "16-byte stores");
     __shared__ float b1[H], b2[H], x[REC][NF], h1[REC][H], h2[REC][H], d1[REC][H], d2[REC][H], dz[REC], dzb[REC];
     const int t = threadIdx.x;
     for (int i = t; i < NF * H / 8; i += THREADS) reinterpret_cast<uint4 *>(w1t)[i] = reinterpret_cast<const uint4 *>(M->w1t)[i];

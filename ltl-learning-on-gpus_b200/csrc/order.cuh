@@ -9,6 +9,7 @@
 // level was exhausted before, so a find is still of minimal cost.
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 
 #include <cuda_bf16.h>
@@ -28,8 +29,9 @@ constexpr int MLP_B3 = MLP_W3 + ORDER_H;             // [1]
 constexpr int MLP_PARAMS = MLP_B3 + 1;
 
 // The scorer on the device: BF16 weights, FP32 biases.  The hidden layers' weights are kept both ways:
-// [out][in], and [in][out] for threads that each compute one unit.
-struct MlpDev {
+// [out][in], and [in][out] for threads that each compute one unit; grad_kernel copies three of them 16
+// bytes at a time.
+struct alignas(16) MlpDev {
     __nv_bfloat16 w1[ORDER_H * ORDER_NF];
     __nv_bfloat16 w2[ORDER_H * ORDER_H];
     __nv_bfloat16 w1t[ORDER_NF * ORDER_H];
@@ -39,6 +41,8 @@ struct MlpDev {
     float b2[ORDER_H];
     float b3;
 };
+static_assert(offsetof(MlpDev, w2) % 16 == 0 && offsetof(MlpDev, w1t) % 16 == 0 && offsetof(MlpDev, w2t) % 16 == 0,
+              "16-byte loads");
 
 // What the features of one block are made of.  Costs are level costs; rows are cache rows.
 // Row statistics of a level: stored rows that hold at position 0 on every positive trace, and
