@@ -7,7 +7,8 @@
 // place in the set (one thread each), then the rows of the new ones written and the matches
 // verified word by word.  Rows and parents go to global memory as everywhere, so the level
 // kernel can take over at any level (local_handoff).  A level is taken only if its candidates
-// could all be new and still fit.
+// could all be new and still fit: this CTA's tables, and the rows and cache that the
+// instance has in the level kernel, so that a search that passes one of those ends as it does there.
 //
 // A learn of 40 short traces to cost 3 took 168 us of which 43 on the device and the rest in launches,
 // copies and waits; with its set-up and levels in this one kernel, one copy down and one back, 80.
@@ -826,7 +827,8 @@ __global__ void __launch_bounds__(LT_BATCH, 2)
             }
             continue;
         }
-        const long long cap = min((long long)LROWS, words / pitch);
+        // as many rows as the CTA's share of the caches holds, and no more than a slot would have
+        const long long cap = min((long long)LROWS, min(min(words, B->cache_words) / pitch, B->max_rows));
         bool over = false;
         if (pitch <= LPITCH && cap > nalpha) {
             if (tid == 0) {
