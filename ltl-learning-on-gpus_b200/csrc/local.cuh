@@ -7,7 +7,7 @@
 // place in the set (one thread each), then the rows of the new ones written and the matches
 // verified word by word.  Rows and parents go to global memory as everywhere, so the level
 // kernel can take over at any level (local_handoff).  A level is taken only if its candidates
-// could all be new and still fit: this CTA's tables, and the rows and cache that the
+// could all be new and still fit: this CTA's tables, and the rows, cache and hash slots that the
 // instance has in the level kernel, so that a search that passes one of those ends as it does there.
 //
 // A learn of 40 short traces to cost 3 took 168 us of which 43 on the device and the rest in launches,
@@ -596,6 +596,8 @@ __device__ bool local_run(Local &S, long long limit, int tid) {
     u64 found = 0;
     int found_cost = 0;
     bool over = false;
+    // rows that fit this CTA and that the instance may have: its row limit, its hash set's slots
+    const u64 room = min((u64)min((long long)LROWS, A.cap_rows), A.slot_mask + 1u);
     if (tid == 0 && A.level_ns) A.level_ns[(u64)c1 * LEVEL_TRACE + LT_END] = globaltimer();
     for (;; ++c) {
         // level c - 1 is complete
@@ -609,7 +611,7 @@ __device__ bool local_run(Local &S, long long limit, int tid) {
             if (lane == 0) {
                 S.found_key = ~0ull;
                 S.ok = (long long)S.units * (its + 1) <= limit &&
-                       (u64)S.nrows + S.cand <= (u64)min((long long)LROWS, A.cap_rows) && !(A.cancel && *A.cancel);
+                       (u64)S.nrows + S.cand <= room && !(A.cancel && *A.cancel);
                 if (S.ok && A.level_ns && S.units) {
                     const u64 t = globaltimer();
                     u64 *ns = A.level_ns + (u64)c * LEVEL_TRACE;

@@ -1,8 +1,10 @@
-"""The engine's limits hold on the small levels too: the rows and cache bytes of the configuration.  A
-search that passes one of them has one answer, whether one CTA ran its small levels
+"""The engine's limits hold on the small levels too: the rows and cache bytes of the configuration, and the
+size of the hash set.  A search that passes one of them has one answer, whether one CTA ran its small levels
 or the level kernel did, alone or in a call of any number of instances."""
+import numpy as np
 import pytest
 
+import oracle as O
 from ltlb200 import api, gen
 from helpers import on_the_fly_cases
 
@@ -33,3 +35,30 @@ def test_batch_calls_of_any_size_keep_the_cache_limits(limit, workers, count, ma
             for n in (3, count):
                 for r in b.learn([inst] * n, neg_type=1, max_cost=max_cost):
                     assert key(r) == key(want), (k, n)
+
+
+# one proposition or two, costs under which many levels are small: 1,095 rows up to cost 19 with at most 200
+# operand pairs in a level; 1,170 up to cost 10 with levels of up to a few thousand candidates
+FULL = [(2, (2, 2, 11, 11, 2, 2, 2, 11), 19, 1), (1, (1, 1, 4, 4, 1, 1, 1, 4), 10, 300)]
+
+
+@pytest.mark.parametrize("props,costs,max_cost,count", FULL)
+def test_full_hash_set_on_small_levels(props, costs, max_cost, count):
+    rng = np.random.default_rng(7)
+    lens, bits, _, _ = gen._draw(rng, 24, props, 8, 30, 0.5)
+    letters = "".join(sorted(gen.DEFAULT_LETTERS[:props]))
+    steps, offs = gen._pack(letters, list(lens), list(bits))
+    inst = gen.Instance(12, 12, letters, steps, offs)
+    opts = dict(costs=costs, max_cost=max_cost, stop_at_found=False, neg_type=1)
+    ref = O.learn(inst, cache_rows=1 << 14, **opts)
+    assert 1024 < ref.num_rows < 2048
+    kw = dict(cache_bytes=64 << 20, max_rows=1 << 15, max_traces=64)
+    for log2, status in ((10, api.TABLE_FULL), (11, None)):
+        with api.Engine(slots_log2=log2, **kw) as e:
+            levels = e.learn(inst, schedule=api.SCHEDULE_PER_BLOCK, **opts)
+            assert status is None or levels.status == status
+            assert e.learn(inst, **opts).status == levels.status
+        with api.Batch(workers=4, slots_log2=log2, **kw) as b:
+            for r in b.learn([inst] * count, **opts):
+                assert r.status == levels.status
+                assert status is not None or r.rows == ref.num_rows
