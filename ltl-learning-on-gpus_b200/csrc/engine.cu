@@ -483,7 +483,8 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
         len_sum += ln;
     }
     // The reference's keys hold whole CSs of up to 126 positions in all (ltli6463.cu:57-73): there they are
-    // exact keys, and the exact path's small levels and fused entries serve them.
+    // exact keys, and the exact path's small levels and fused entries serve them, with the reference's order
+    // (prio) deciding which candidate a CS's row has its parents from.
     const int key_mode = opt->key_mode == LTLG_KEY_REF && len_sum <= 126 ? (int)LTLG_KEY_EXACT : opt->key_mode;
     const bool ref_keys = key_mode == LTLG_KEY_REF;
     res->cost = c1;
@@ -601,7 +602,8 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
     if ((err = ensure(e->parents, (size_t)cap_rows * 8)) != cudaSuccess) return fail_cuda(e, err, res);
     if (key_mode != LTLG_KEY_EXACT && (err = ensure(e->keys, (size_t)cap_rows * 16)) != cudaSuccess)
         return fail_cuda(e, err, res);
-    if (ref_keys && (err = ensure(e->prio, (size_t)cap_rows * 8)) != cudaSuccess) return fail_cuda(e, err, res);
+    const bool ordered = opt->key_mode == LTLG_KEY_REF;
+    if (ordered && (err = ensure(e->prio, (size_t)cap_rows * 8)) != cudaSuccess) return fail_cuda(e, err, res);
     const Down dl(ncost);
     if ((err = ensure(e->wmeta, (size_t)pitch * 8)) != cudaSuccess || (err = ensure(e->ne, (size_t)ncost * 4)) != cudaSuccess ||
         (err = ensure(e->lstats, (size_t)ncost * LSTATS * 8)) != cudaSuccess ||
@@ -652,7 +654,7 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
     A.cache = (u64 *)e->cache.p;
     A.parents = (u64 *)e->parents.p;
     A.keys = key_mode != LTLG_KEY_EXACT ? (u64 *)e->keys.p : nullptr;
-    A.prio = ref_keys ? (u64 *)e->prio.p : nullptr;
+    A.prio = ordered ? (u64 *)e->prio.p : nullptr;
     A.slots = (u64 *)e->slots.p;
     A.wmeta = (const u64 *)e->wmeta.p;
     A.kmeta = (const u32 *)(du + upl.kmeta);

@@ -30,7 +30,7 @@
 // Semantics follow MojtabaValizadeh/ltl-learning-on-gpus, code/ltli6463.cu:
 //   acceptance ......... :240-243 (positives need bit 0 set, negatives clear)
 //   uniqueness ......... :224-231 (a candidate is stored iff its key is new)
-//   relaxed keys ....... :57-141 (KEY_REF, types 1/2/3 and the exact 126-bit pack)
+//   relaxed keys ....... :57-141 (KEY_REF, types 1/2/3; up to 126 positions the key is the whole CS)
 //   level / block order  :1199-1445 (NegType rule :1212)
 // Every device wait is bounded; giving up sets a status bit the host reads.
 #include <atomic>
@@ -376,19 +376,13 @@ __device__ __noinline__ void count_one_row(const InstArgs &A, int cost, const ul
     count_stats(A.lstats + (u64)cost * LSTATS, !__any_sync(FULL, pm), !__any_sync(FULL, nh), lane);
 }
 
-// Lane t owns candidate t (t < NC).  Claims are written and
-// published before any lane waits on another warp's publication, so waits cannot cycle.
-// Lane t owns candidate t (t < NC).  Every phase that touches whole CSs (writing the
-// claimed rows, verifying fingerprint matches) is one chunk-major sweep over all the
-// candidates concerned, so their loads are in flight together.  Claims are written and
-// published before any lane waits on another warp's publication, so waits cannot cycle.
-// The reference's relaxed keys keep, of the CSs that share a key in a level, the one its
+// The reference's keys keep, of the candidates that share a key in a level, the one its
 // threads insert first: blocks run in order and, within a block, roughly thread order (the
 // oracle's sequential tid order).  Here the row of a key records the priority (block position
 // << 40 | the reference's thread index, U's "l U r" before "r U l") of the candidate it holds;
 // a candidate of the same level with the same key and a lower priority takes the row over: it
-// locks the priority word (bit 0), rewrites the row and its parent, and publishes its
-// priority.  Rows of lower levels are never taken over.  So a shared key never goes to a later
+// locks the priority word (bit 0), rewrites the row (where the key is not the whole CS) and its
+// parent, and publishes its priority.  Rows of lower levels are never taken over.  So a shared key never goes to a later
 // block, which keeps the per-block stored counts equal to the oracle's; inside a block the
 // thread index counts operand rows in the order they were stored, which on the device (as in
 // the reference) is the order warps reached the hash set.  One lane, bounded waits.
@@ -405,7 +399,8 @@ __device__ void take_over(const InstArgs &A, InstCtl *C, const Gen &g, int t, u6
         }
         if (atomicCAS(pw, v, (prio << 1) | 1ull) != v) continue;
         ulonglong2 *dst = reinterpret_cast<ulonglong2 *>(A.cache + row * (u64)A.pitch);
-        for (int c = 0; c < nch; ++c) dst[c] = g.word(t, c, g.pre(c));
+        if (A.key_mode == KEY_REF)
+            for (int c = 0; c < nch; ++c) dst[c] = g.word(t, c, g.pre(c));
         A.parents[row] = parent;
         __threadfence();
         st_release(pw, prio << 1);
@@ -414,6 +409,10 @@ __device__ void take_over(const InstArgs &A, InstCtl *C, const Gen &g, int t, u6
     atomicOr(&C->status, ST_WAIT);
 }
 
+// Lane t owns candidate t (t < NC).  Every phase that touches whole CSs (writing the
+// claimed rows, verifying fingerprint matches) is one chunk-major sweep over all the
+// candidates concerned, so their loads are in flight together.  Claims are written and
+// published before any lane waits on another warp's publication, so waits cannot cycle.
 template <int NC, bool WIDE, class Gen>
 __device__ __forceinline__ void resolve(const InstArgs &A, InstCtl *C, int cost, const Gen &g, u64 fp, bool active,
                                         u64 parent, u64 kh, u64 kl, u64 prio, u32 anyp, u32 anyn, int *overflowed,
@@ -541,6 +540,7 @@ __device__ __forceinline__ void resolve(const InstArgs &A, InstCtl *C, int cost,
             }
         }
         // Verification of fingerprint matches: one sweep comparing every candidate with its row.
+        bool same = false;
         if (A.key_mode == KEY_EXACT) {
             const u32 vm = __ballot_sync(FULL, state == S_VERIFY);
             if (vm) {
@@ -582,25 +582,28 @@ __device__ __forceinline__ void resolve(const InstArgs &A, InstCtl *C, int cost,
                         idx = (idx + 1) & mask;
                     } else {
                         state = S_DONE;
+                        same = true;
                     }
                 }
             }
         } else if (state == S_VERIFY) {
             const u64 eh = __ldcg(A.keys + 2 * vrow), el = __ldcg(A.keys + 2 * vrow + 1);
             if (eh == kh && el == kl) {
-                if (A.prio && vrow >= __ldcg(A.ls + cost)) take_over(A, C, g, lane, (u64)vrow, prio, parent);
                 state = S_DONE;
+                same = true;
             } else {
                 state = S_PROBE;
                 idx = (idx + 1) & mask;
             }
         }
+        if (A.prio && same && vrow >= __ldcg(A.ls + cost)) take_over(A, C, g, lane, (u64)vrow, prio, parent);
     }
 }
 
 // Whether a candidate's CS is one that the level's other candidates or the levels below are known to
 // store, from how its operand rows were made (their parents), so that it needs no probe and no
-// comparison.  Exact keys only: a relaxed key may have dropped the row an identity leads to.  Every
+// comparison.  Exact keys only: a relaxed key may have dropped the row an identity leads to; and not under
+// the reference's, where the candidate may be the one in the level's first block that gives the row its parents.  Every
 // identity is one of finite-trace LTL, valid word by word, and leads to
 //   - a stored row (one of the operands, a row below), or
 //   - a candidate of lower cost under any operator costs (that level is complete), or
@@ -705,7 +708,7 @@ __device__ __forceinline__ void finish(const InstArgs &A, InstCtl *C, Slot &sl, 
     // no hash slots
     const bool room = *(volatile int *)&sl.overflowed == 0;
     bool mine = room && ((valid >> lane) & 1u) != 0u;
-    if (A.key_mode == KEY_EXACT && A.pitch >= KNOWN_PITCH && mine) {
+    if (A.key_mode == KEY_EXACT && !A.prio && A.pitch >= KNOWN_PITCH && mine) {
         const int op = parent_op(myparent);
         const u32 x = (u32)parent_left(myparent), y = (u32)parent_right(myparent);
         const bool un = op == OP_NEG || op == OP_X || op == OP_F || op == OP_G;

@@ -206,6 +206,14 @@ __device__ __forceinline__ u64 local_parent(const LocalUnit &x, int t) {
     return mode_swapped(M_ALL, t) ? pack_parent(OP_U, (u64)x.r, (u64)x.l)
                                   : pack_parent(mode_op(M_ALL, t, 0), (u64)x.l, (u64)x.r);
 }
+// Its place in the reference's order, as the level kernel's A.prio has it: block position << 40 | the reference's
+// thread index (U: l U r before r U l).
+__device__ __forceinline__ u64 local_prio(const LocalUnit &x, int t) {
+    const LocalSeg &g = *x.g;
+    const u64 pair = g.mode == M_UNARY ? (u64)(x.r - g.r0) : (u64)(x.l - g.l0) * (u64)g.nr + (u64)(x.r - g.r0);
+    const bool until = g.mode != M_UNARY && mode_op(M_ALL, t, 0) == OP_U;
+    return ((u64)(u32)g.upos[t] << 40) | (until ? 2 * pair + (mode_swapped(M_ALL, t) ? 1u : 0u) : pair);
+}
 // What a candidate is made of: its operand rows (unary: right only) and its operator (W_URL, or a code).
 // & | U are one formula on a = l | r under word masks: a & ((y & (l | n)) | (~(a + y) & u) | o), y the
 // operand U reaches (r, or l for r U l), so that one loop without branches serves them.
@@ -427,6 +435,7 @@ __device__ void local_level(Local &S, int c, int tid) {
                     if (gl == 0) {
                         S.tab[S.idx[j]] = (unsigned short)(at + 1u);
                         A.parents[at] = local_parent(x, j & 3);
+                        if (A.prio) A.prio[at] = local_prio(x, j & 3) << 1;
                         if (A.keys) {
                             A.keys[2 * (u64)at] = S.sum[j];
                             A.keys[2 * (u64)at + 1] = 0;
@@ -454,11 +463,28 @@ __device__ void local_level(Local &S, int c, int tid) {
                 }
             }
             __syncthreads();
+            // (the reference's keys: a match in a row of this level gives it its parents if it comes first in the
+            // reference's order)
+            auto row_of = [&](int j) {
+                const u32 at = S.at[j];
+                return at & LMATCH ? S.at[at & ~LMATCH] : at;
+            };
             for (int i = tid; i < n - nc; i += LT) {
                 const int j = S.verify[i];
-                if (S.fail[j]) S.retry[p][atomicAdd(&S.nretry[p], 1u)] = (unsigned short)j;
+                if (S.fail[j])
+                    S.retry[p][atomicAdd(&S.nretry[p], 1u)] = (unsigned short)j;
+                else if (A.prio && (int)row_of(j) >= S.ls[c])
+                    atomicMin(A.prio + row_of(j), local_prio(local_unit(S, j >> 2), j & 3) << 1);
             }
             __syncthreads();
+            if (A.prio)
+                for (int i = tid; i < n - nc; i += LT) {
+                    const int j = S.verify[i];
+                    if (S.fail[j] || (int)row_of(j) < S.ls[c]) continue;
+                    const LocalUnit x = local_unit(S, j >> 2);
+                    if (ld_volatile(A.prio + row_of(j)) == local_prio(x, j & 3) << 1)
+                        A.parents[row_of(j)] = local_parent(x, j & 3);
+                }
             const int nr = (int)S.nretry[p];
             if (tid == 0) {
                 S.nclaim = 0;

@@ -149,7 +149,7 @@ struct InstArgs {
     int npos;
     int nalpha;
     int key_mode;
-    int rlx_type;        // KEY_REF: 0 exact pack, 1, 2, 3
+    int rlx_type;        // KEY_REF: 1, 2, 3
     int stop_at_found;
     int find_first;      // 1: any find stops the level; 0: the first block of the reference's order that holds one
     int neg_type;
@@ -172,7 +172,8 @@ struct InstArgs {
     u64 *cache;
     u64 *parents;
     u64 *keys;           // 2 words per row for KEY_REF / KEY_HASH64, else null
-    u64 *prio;           // KEY_REF: per row, the priority of the candidate it holds << 1 | lock (else null)
+    u64 *prio;           // the reference's keys (KEY_REF, and exact ones in their place): per row, the priority of the
+                         // candidate it holds << 1 | lock (else null)
     u64 *slots;
     const u64 *wmeta;    // per word: length mask | (positive << 63); 0 for padding
     const u32 *kmeta;    // KEY_REF: per word start | count << 16 | step << 24
