@@ -702,7 +702,7 @@ LTLG_API int ltlg_engine_learn(ltlg_engine *e, const ltlg_traces *t, const ltlg_
     e->held = false;
     if (persist && !held && local_takes(A.key_mode, pitch)) {
         // set-up and the small levels on one CTA
-        if ((err = launch_start(dA, din, hk, st)) != cudaSuccess) return fail_cuda(e, err, res);
+        if ((err = launch_start(dA, din, hk, ordered, st)) != cudaSuccess) return fail_cuda(e, err, res);
         o.launches = 1;
     } else {
         if ((err = launch_init(dA, din, pitch, st)) != cudaSuccess) return fail_cuda(e, err, res);

@@ -2361,7 +2361,7 @@ cudaError_t launch_init(const InstArgs *d, const StartIn *in, int pitch, cudaStr
 
 bool local_takes(int key_mode, int pitch) { return key_mode != KEY_REF && pitch <= LPITCH; }
 
-template <int HK>
+template <int HK, bool TIES>
 static cudaError_t launch_start_hk(const InstArgs *d, const StartIn *in, cudaStream_t s) {
     // the shared-memory limit is a per-device attribute of the kernel: set once on each device
     static std::atomic<unsigned long long> done{0};
@@ -2369,11 +2369,11 @@ static cudaError_t launch_start_hk(const InstArgs *d, const StartIn *in, cudaStr
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev >= 64 || !((done.load() >> dev) & 1ull)) {
-        e = cudaFuncSetAttribute(start_kernel<HK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Local));
+        e = cudaFuncSetAttribute(start_kernel<HK, TIES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Local));
         if (e != cudaSuccess) return e;
         if (dev < 64) done.fetch_or(1ull << dev);
     }
-    start_kernel<HK><<<1, LT_ONE, sizeof(Local), s>>>(d, in, LOCAL_LEVEL_WORK);
+    start_kernel<HK, TIES><<<1, LT_ONE, sizeof(Local), s>>>(d, in, LOCAL_LEVEL_WORK);
     return cudaGetLastError();
 }
 
@@ -2392,8 +2392,10 @@ cudaError_t launch_batch_local(BatchDev *d, const InstArgs *args, long long word
                    : launch_batch_local_hk<0>(d, args, words, limit, ctas, s);
 }
 
-cudaError_t launch_start(const InstArgs *d, const StartIn *in, int hk, cudaStream_t s) {
-    return hk == 1 ? launch_start_hk<1>(d, in, s) : launch_start_hk<0>(d, in, s);
+cudaError_t launch_start(const InstArgs *d, const StartIn *in, int hk, bool ties, cudaStream_t s) {
+    return hk == 1 ? launch_start_hk<1, false>(d, in, s)
+           : ties  ? launch_start_hk<0, true>(d, in, s)
+                   : launch_start_hk<0, false>(d, in, s);
 }
 
 cudaError_t launch_plan_level(const InstArgs *d, int cost, cudaStream_t s) {

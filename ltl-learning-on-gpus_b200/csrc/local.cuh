@@ -206,14 +206,6 @@ __device__ __forceinline__ u64 local_parent(const LocalUnit &x, int t) {
     return mode_swapped(M_ALL, t) ? pack_parent(OP_U, (u64)x.r, (u64)x.l)
                                   : pack_parent(mode_op(M_ALL, t, 0), (u64)x.l, (u64)x.r);
 }
-// Its place in the reference's order, as the level kernel's A.prio has it: block position << 40 | the reference's
-// thread index (U: l U r before r U l).
-__device__ __forceinline__ u64 local_prio(const LocalUnit &x, int t) {
-    const LocalSeg &g = *x.g;
-    const u64 pair = g.mode == M_UNARY ? (u64)(x.r - g.r0) : (u64)(x.l - g.l0) * (u64)g.nr + (u64)(x.r - g.r0);
-    const bool until = g.mode != M_UNARY && mode_op(M_ALL, t, 0) == OP_U;
-    return ((u64)(u32)g.upos[t] << 40) | (until ? 2 * pair + (mode_swapped(M_ALL, t) ? 1u : 0u) : pair);
-}
 // What a candidate is made of: its operand rows (unary: right only) and its operator (W_URL, or a code).
 // & | U are one formula on a = l | r under word masks: a & ((y & (l | n)) | (~(a + y) & u) | o), y the
 // operand U reaches (r, or l for r U l), so that one loop without branches serves them.
@@ -336,9 +328,23 @@ __device__ __forceinline__ void local_probe(Local &S, int j, u32 idx) {
     }
 }
 
+// Its place in the reference's order, as the level kernel's A.prio has it: block position << 40 | the reference's
+// thread index (U: l U r before r U l).
+__device__ __forceinline__ u64 local_prio(const LocalUnit &x, int t) {
+    const LocalSeg &g = *x.g;
+    const u64 pair = g.mode == M_UNARY ? (u64)(x.r - g.r0) : (u64)(x.l - g.l0) * (u64)g.nr + (u64)(x.r - g.r0);
+    const bool until = g.mode != M_UNARY && mode_op(M_ALL, t, 0) == OP_U;
+    return ((u64)(u32)g.upos[t] << 40) | (until ? 2 * pair + (mode_swapped(M_ALL, t) ? 1u : 0u) : pair);
+}
+// The row that candidate j of the round stands for: its own, or the one it matches.
+__device__ __forceinline__ int local_row(const Local &S, int j) {
+    const u32 at = S.at[j];
+    return (int)(at & LMATCH ? S.at[at & ~LMATCH] : at);
+}
+
 // One level, already planned, by the whole CTA.  Returns with the level's rows stored, nrows and
-// the find updated.
-template <int HK, int LT>
+// the find updated.  TIES: the reference's keys, kept out of the other learns' code (40 traces: 1.8% longer with it).
+template <int HK, int LT, bool TIES>
 __device__ void local_level(Local &S, int c, int tid) {
     const int lane = tid & 31, warp = tid >> 5;
     const InstArgs &A = S.A;
@@ -435,7 +441,7 @@ __device__ void local_level(Local &S, int c, int tid) {
                     if (gl == 0) {
                         S.tab[S.idx[j]] = (unsigned short)(at + 1u);
                         A.parents[at] = local_parent(x, j & 3);
-                        if (A.prio) A.prio[at] = local_prio(x, j & 3) << 1;
+                        if (TIES) A.prio[at] = local_prio(x, j & 3) << 1;
                         if (A.keys) {
                             A.keys[2 * (u64)at] = S.sum[j];
                             A.keys[2 * (u64)at + 1] = 0;
@@ -463,27 +469,20 @@ __device__ void local_level(Local &S, int c, int tid) {
                 }
             }
             __syncthreads();
-            // (the reference's keys: a match in a row of this level gives it its parents if it comes first in the
-            // reference's order)
-            auto row_of = [&](int j) {
-                const u32 at = S.at[j];
-                return at & LMATCH ? S.at[at & ~LMATCH] : at;
-            };
             for (int i = tid; i < n - nc; i += LT) {
                 const int j = S.verify[i];
                 if (S.fail[j])
                     S.retry[p][atomicAdd(&S.nretry[p], 1u)] = (unsigned short)j;
-                else if (A.prio && (int)row_of(j) >= S.ls[c])
-                    atomicMin(A.prio + row_of(j), local_prio(local_unit(S, j >> 2), j & 3) << 1);
+                else if (TIES && local_row(S, j) >= S.ls[c])
+                    atomicMin(A.prio + local_row(S, j), local_prio(local_unit(S, j >> 2), j & 3) << 1);
             }
             __syncthreads();
-            if (A.prio)
+            if (TIES)  // of the candidates in one row of the level, the first in the reference's order gives its parents
                 for (int i = tid; i < n - nc; i += LT) {
-                    const int j = S.verify[i];
-                    if (S.fail[j] || (int)row_of(j) < S.ls[c]) continue;
+                    const int j = S.verify[i], row = local_row(S, j);
                     const LocalUnit x = local_unit(S, j >> 2);
-                    if (ld_volatile(A.prio + row_of(j)) == local_prio(x, j & 3) << 1)
-                        A.parents[row_of(j)] = local_parent(x, j & 3);
+                    if (!S.fail[j] && row >= S.ls[c] && ld_volatile(A.prio + row) == local_prio(x, j & 3) << 1)
+                        A.parents[row] = local_parent(x, j & 3);
                 }
             const int nr = (int)S.nretry[p];
             if (tid == 0) {
@@ -612,7 +611,7 @@ __device__ void local_begin(Local &S, int tid) {
 // 32-chunk steps + 1).  On return the control block and the level arrays stand as before the closing
 // of the last complete level (plan.cost), which close_level does; returns true when that will end
 // the search, false when the next level is for the level kernel.
-template <int HK, int LT>
+template <int HK, int LT, bool TIES>
 __device__ bool local_run(Local &S, long long limit, int tid) {
     const InstArgs &A = S.A;
     InstCtl *C = A.ctl;
@@ -652,7 +651,7 @@ __device__ bool local_run(Local &S, long long limit, int tid) {
             if (S.ls[c] > S.ls[c - 1]) A.ne[ne] = c - 1;
         }
         if (S.ls[c] > S.ls[c - 1]) ++ne;
-        if (S.units) local_level<HK, LT>(S, c, tid);
+        if (S.units) local_level<HK, LT, TIES>(S, c, tid);
         __syncthreads();
         if (S.found_key != ~0ull && !found) {
             found = (1ull << 63) | S.found_parent;
@@ -710,7 +709,7 @@ __device__ void local_handoff(Local &S, int tid) {
 
 // One instance from its traces: set-up, the small levels, and the plan of the first level that is
 // left to the level kernel (or the end of the search).
-template <int HK>
+template <int HK, bool TIES>
 __global__ void __launch_bounds__(LT_ONE, 1)
     start_kernel(const InstArgs *__restrict__ args, const StartIn *__restrict__ in, long long limit) {
     constexpr int LT = LT_ONE;
@@ -724,7 +723,7 @@ __global__ void __launch_bounds__(LT_ONE, 1)
     init_state(S.A, tid, LT);
     __syncthreads();
     local_begin<HK, LT>(S, tid);
-    if (!local_run<HK, LT>(S, limit, tid)) local_handoff<LT>(S, tid);
+    if (!local_run<HK, LT, TIES>(S, limit, tid)) local_handoff<LT>(S, tid);
     __threadfence();
     __syncthreads();
     if (tid < 32) close_level(S.A, S.A.ctl, true, tid);
@@ -879,7 +878,7 @@ __global__ void __launch_bounds__(LT_BATCH, 2)
             init_traces(S.A, in, S.meta, tid, LT);
             __syncthreads();
             local_begin<HK, LT>(S, tid);
-            over = local_run<HK, LT>(S, limit, tid);
+            over = local_run<HK, LT, false>(S, limit, tid);
         }
         if (tid < 32) {
             if (over)

@@ -313,9 +313,9 @@ struct StartIn {
 // Set-up of an instance (letters, word metadata, level arrays, control block) from its traces.
 cudaError_t launch_init(const InstArgs *d, const StartIn *in, int pitch, cudaStream_t s);
 // Set-up, the small levels on one CTA, and the plan of the first larger level (csrc/local.cuh); only
-// where local_takes says so.
+// where local_takes says so.  ties: exact keys in place of the reference's (InstArgs::prio).
 bool local_takes(int key_mode, int pitch);
-cudaError_t launch_start(const InstArgs *d, const StartIn *in, int hash_kind, cudaStream_t s);
+cudaError_t launch_start(const InstArgs *d, const StartIn *in, int hash_kind, bool ties, cudaStream_t s);
 // The instances of a batch that end on small levels, one per CTA (args: per CTA, `words` words of rows each).
 constexpr int LOCAL_BATCH_FACTOR = 12;  // how much larger levels a CTA takes when every SM has instances
 constexpr int LOCAL_ROWS = 5120;  // rows a CTA takes an instance to
