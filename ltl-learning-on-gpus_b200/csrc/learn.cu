@@ -69,7 +69,7 @@ struct Slot {
     int upos[4];              // unary: block position of each slot operator; fused binary: of & | U
     int cost;
     int check_only;
-    int stop;                 // remaining rows are skipped (a find at or before this entry)
+    int live;                 // operators of the entry still to run (live_ops); 0: remaining rows are skipped
     int inst;                 // the item's instance (index into Launch::args)
     int trace_first;          // the producer's first item of this plan (level stamps)
     int split;                // units per row (left groups of the tile; a small level's unary operators)
@@ -80,6 +80,17 @@ struct Slot {
     InstArgs args;            // its arguments as they were when the item was claimed (a batch slot's
                               // arguments change when it takes the next instance)
 };
+
+// How many of an entry's operators are still worth running once the level has a find in block `found`: those whose
+// block comes before it (find_first: none), which are the first ones, as a fused entry's blocks & | U come in this
+// order.  Other entries go on as a whole or not at all (a fused unary entry until its first block is passed).
+__host__ __device__ __forceinline__ int entry_ops(int kind) { return kind == ENT_ALL ? 3 : kind == ENT_AO ? 2 : 1; }
+__device__ __forceinline__ int live_ops(int kind, int pos, const int (&upos)[4], int found, bool find_first) {
+    if (find_first || pos >= found) return 0;
+    int n = 1;
+    while (n < entry_ops(kind) && upos[n] < found) ++n;
+    return n;
+}
 
 // ---------------------------------------------------------------- candidate generators
 // pre(c) loads everything of chunk c that the set's candidates read from global memory
@@ -681,8 +692,9 @@ __device__ __forceinline__ void finish(const InstArgs &A, InstCtl *C, Slot &sl, 
                 atomicCAS(A.found_par + p, 0ull, (1ull << 63) | myparent);
                 atomicMin(&C->found_key, key);
             }
-            // the item's remaining rows are skipped only when the search ends at this level
-            if (A.stop_at_found && (A.find_first || sl.pos >= p)) sl.stop = 1;
+            // the item's remaining rows are skipped, or run under fewer operators, only when the search ends
+            // at this level
+            if (A.stop_at_found) atomicMin(&sl.live, live_ops(sl.kind, sl.pos, sl.upos, p, A.find_first != 0));
         }
         __syncwarp();
         if (A.stop_at_found) return;  // this level is the last one; its candidates need no dedupe
@@ -1646,13 +1658,15 @@ __device__ __noinline__ void next_instance(BatchDev &B, int s, bool finishing, i
 __device__ __forceinline__ Slot *slot_at(unsigned char *smem, int s) { return reinterpret_cast<Slot *>(smem) + s; }
 
 // Item `item` of entry e (cached in shared memory) into slot sl.  Returns the tile bytes to copy
-// (0 for a unary item or a skipped one).
+// (0 for a unary item or a skipped one).  `live` of the entry's operators are run.
 __device__ __forceinline__ u32 fill_slot(Slot &sl, int inst, const Entry &e, long long item, int tile, int rc,
-                                         int ur, int cost, int check_only, long long plan_items, bool skip,
+                                         int ur, int cost, int check_only, long long plan_items, int live,
                                          int pitch) {
     const long long local = item - e.item0;
+    const bool skip = live == 0;
     sl.inst = inst;
-    sl.kind = e.kind;
+    // a fused entry of which only & | or & are left is the smaller entry of these
+    sl.kind = skip || live == entry_ops(e.kind) ? e.kind : live == 2 ? (int)ENT_AO : (int)ENT_ONE;
     sl.pos = e.pos;
     for (int j = 0; j < 4; ++j) sl.upos[j] = e.upos[j];
     sl.cost = cost;
@@ -1661,7 +1675,7 @@ __device__ __forceinline__ u32 fill_slot(Slot &sl, int inst, const Entry &e, lon
     sl.next_row = 0;
     sl.rows_done = 0;
     sl.evals = 0;
-    sl.stop = skip ? 1 : 0;
+    sl.live = live;
     sl.e_l0 = e.l0;
     sl.e_r0 = e.r0;
     sl.e_R = e.r1 - e.r0;
@@ -1879,16 +1893,18 @@ __device__ void producer(const Launch &L, unsigned char *smem, u64 *tiles, int l
             if (lane == 0) pc.cur = lo;
             __syncwarp();
         }
-        // skip rule: a find at or before this entry's block (or any find, find_first) in this level
+        // skip rule: operators whose block comes after a find of this level (or any find, find_first)
         const bool found_here = pc.a.stop_at_found && fk != NO_FIND && (int)(fk >> 32) == pc.cost;
-        const bool skip = found_here && (pc.a.find_first || pc.e.pos >= (int)(u32)fk);
-        // the same rule for the items of this level still in this CTA's slots: their remaining
-        // rows are skipped (the slot the producer is about to fill is not in flight)
+        const int live = found_here ? live_ops(pc.e.kind, pc.e.pos, pc.e.upos, (int)(u32)fk, pc.a.find_first != 0)
+                                    : entry_ops(pc.e.kind);
+        const bool skip = live == 0;
+        // the same rule for the remaining rows of the items of this level still in this CTA's slots (the slot
+        // the producer is about to fill is not in flight)
         if (found_here && lane < S && lane != s) {
             Slot &o = *slot_at(smem, lane);
-            if (*(volatile int *)&o.kind != 0 && o.inst == inst && o.cost == pc.cost &&
-                (pc.a.find_first || o.pos >= (int)(u32)fk))
-                *(volatile int *)&o.stop = 1;
+            const int kind = *(volatile int *)&o.kind;
+            if (kind != 0 && o.inst == inst && o.cost == pc.cost)
+                atomicMin(&o.live, live_ops(kind, o.pos, o.upos, (int)(u32)fk, pc.a.find_first != 0));
         }
         {
             constexpr int AW = sizeof(InstArgs) / 8;
@@ -1898,7 +1914,7 @@ __device__ void producer(const Launch &L, unsigned char *smem, u64 *tiles, int l
         }
         if (lane == 0) {
             const u32 bytes = fill_slot(sl, inst, pc.e, item, L.tile, pc.rc, pc.ur, pc.cost, pc.check_only,
-                                        pc.plan_items, skip, pc.a.pitch);
+                                        pc.plan_items, live, pc.a.pitch);
             sl.trace_first = pc.trace_first;
             sl.overflowed = ovf ? 1 : 0;
             // units: a right row with unit_lefts of the tile's left rows; at a small level one left
@@ -1968,7 +1984,8 @@ __device__ __forceinline__ int take_rows(Slot &sl, int kind, const ulonglong2 *t
         if ((int)idx >= sl.units) break;
         if (idx == 0 && sl.trace_first && lane == 0)
             atomicCAS(A.level_ns + (u64)sl.cost * LEVEL_TRACE + LT_STARTED, 0ull, globaltimer());
-        if (!*(volatile int *)&sl.stop) {
+        const int live = __shfl_sync(FULL, *(volatile int *)&sl.live, 0);
+        if (live) {
             const int split = sl.split, part = (int)idx % split;
             const long long r = sl.row0 + (int)idx / split;
             const ulonglong2 *rp = reinterpret_cast<const ulonglong2 *>(A.cache + (u64)r * A.pitch);
@@ -1981,9 +1998,9 @@ __device__ __forceinline__ int take_rows(Slot &sl, int kind, const ulonglong2 *t
                 const ulonglong2 *t0 = tile + (u64)first * (u64)nch;
                 const int nl = min(sl.lefts, sl.nl - first);
                 const long long lf = sl.l_first + first;
-                if (kind == ENT_ALL)
+                if (kind == ENT_ALL && live == 3)
                     binary_unit<M_ALL, unit_lefts<TL>(M_ALL), HK, WIDE>(A, C, sl, t0, nl, lf, rp, r, ring, lane);
-                else if (kind == ENT_AO)
+                else if ((kind == ENT_ALL || kind == ENT_AO) && live == 2)
                     binary_unit<M_AO, unit_lefts<TL>(M_AO), HK, WIDE>(A, C, sl, t0, nl, lf, rp, r, ring, lane);
                 else if (kind == ENT_U)
                     binary_unit<M_U, unit_lefts<TL>(M_U), HK, WIDE>(A, C, sl, t0, nl, lf, rp, r, ring, lane);

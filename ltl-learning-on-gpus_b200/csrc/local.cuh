@@ -56,6 +56,7 @@ struct Local {
     u64 found_key;             // smallest block position << 32 | candidate of the level
     u64 found_parent;
     u64 evaluated;
+    u32 skipped;               // candidates of the level behind its find
     int ok;
     u32 every, some;           // batches: letters that hold first in every positive / some negative
 };
@@ -354,6 +355,10 @@ __device__ void local_level(Local &S, int c, int tid) {
     const int gl = lane & (P - 1), per_warp = 32 / P, group = tid / P, ngroups = LT / P;
     for (int u0 = 0; u0 < S.units; u0 += LC / 4) {
         const int nu = min(LC / 4, S.units - u0);
+        // Once a round has found and the search ends here, the later ones run the operators whose blocks come
+        // before the find, for acceptance only: nothing of the level is an operand any more.
+        const bool over = A.stop_at_found && S.found_key != ~0ull;
+        const int found = (int)(S.found_key >> 32);
         if (tid < nu) local_decode(S, tid, u0 + tid);
         __syncthreads();
         // fingerprints and acceptance
@@ -364,9 +369,15 @@ __device__ void local_level(Local &S, int c, int tid) {
             if (u < nu) {
                 const LocalUnit x = local_unit(S, u);
                 valid = (u32)x.g->op;
-                if (x.g->mode == M_UNARY)
+                if (over) {
+#pragma unroll
+                    for (int t = 0; t < 4; ++t)
+                        if (x.g->upos[t] >= found) valid &= ~(1u << t);
+                    if (gl == 0) atomicAdd(&S.skipped, (u32)__popc((u32)x.g->op & ~valid));
+                }
+                if (valid && x.g->mode == M_UNARY)
                     local_eval<M_UNARY, HK>(S, x, gl, P, h, fails);
-                else
+                else if (valid)
                     local_eval<M_ALL, HK>(S, x, gl, P, h, fails);
             }
             __syncwarp();
@@ -403,6 +414,7 @@ __device__ void local_level(Local &S, int c, int tid) {
                 atomicMin(&S.found_key, mine[q]);
                 if (A.stop_at_found) continue;  // the last level: no dedupe
             }
+            if (over) continue;
             local_probe(S, j, (u32)S.sum[j] & (LTAB - 1));
         }
         __syncthreads();
@@ -635,6 +647,7 @@ __device__ bool local_run(Local &S, long long limit, int tid) {
             local_plan(S, c, lane);
             if (lane == 0) {
                 S.found_key = ~0ull;
+                S.skipped = 0;
                 S.ok = (long long)S.units * (its + 1) <= limit &&
                        (u64)S.nrows + S.cand <= room && !(A.cancel && *A.cancel);
                 if (S.ok && A.level_ns && S.units) {
@@ -661,7 +674,7 @@ __device__ bool local_run(Local &S, long long limit, int tid) {
         for (int k = c + 1 + tid; k < LCOST + 3; k += LT) S.ls[k] = (int)S.nrows;
         if (tid == 0) {
             A.level_cands[c] = S.lc[c] = S.cand;
-            S.evaluated += S.cand;
+            S.evaluated += S.cand - S.skipped;
             if (A.level_ns) A.level_ns[(u64)c * LEVEL_TRACE + LT_END] = globaltimer();
         }
         __syncthreads();
