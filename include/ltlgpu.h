@@ -154,7 +154,8 @@ typedef struct ltlg_result {
     int64_t rows;              /* rows in the language cache (letters included) */
     char *formula;             /* the reference's string format, or its sentinel text */
     double seconds;            /* host wall time of the call */
-    double device_ms;          /* device time of the level loop */
+    double device_ms;          /* device time of set-up and levels; in a batch, the time spent on this
+                                  instance (others run beside it) */
     int32_t num_levels;
     int32_t num_blocks;
     ltlg_level_stat *levels;

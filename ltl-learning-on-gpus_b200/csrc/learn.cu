@@ -1473,7 +1473,7 @@ __device__ bool setup_instance(BatchDev &B, int s, int idx, int lane) {
     const int c1 = A.cf[0];
     if (lane == 0) {
         B.cur[s] = idx;
-        B.t0[s] = globaltimer();
+        B.t0[s] = globaltimer() - (B.order ? o.ns : 0ull);  // what a CTA's pass over its small levels took counts
         o.letter = -1;
         o.walk_count = 0;
         o.walk_overflow = 0;

@@ -894,10 +894,12 @@ __global__ void __launch_bounds__(LT_BATCH, 2)
             over = local_run<HK, LT, false>(S, limit, tid);
         }
         if (tid < 32) {
-            if (over)
+            if (over) {
                 local_result(S, o, t0, hit, lane);
-            else if (lane == 0)
+            } else if (lane == 0) {
+                o.ns = globaltimer() - t0;
                 B->order[atomicAdd(&B->pending, 1)] = idx;
+            }
         }
     }
 }

@@ -214,7 +214,8 @@ struct BatchOut {              // one instance's result
     int walk_count;            // entries of walk: (row, parents), breadth first, entry 0 the root
     int walk_overflow;         // 1: the tree has more entries than the reference prints
     u32 device_flags;
-    u64 ns;                    // device time from the slot's set-up to the result (globaltimer)
+    u64 ns;                    // device time on the instance (globaltimer): a CTA's pass over its small levels,
+                               // and its slot from set-up to the result
     u64 walk[2 * WALK_MAX];
 };
 
@@ -225,7 +226,7 @@ struct BatchDev {
     BatchOut *out;
     InstArgs *args;            // per slot (the slot's buffers and the learn's options; set-up fills the rest)
     int *cur;                  // per slot: the instance it holds
-    u64 *t0;                   // per slot: globaltimer at its set-up
+    u64 *t0;                   // per slot: globaltimer at its set-up, less the instance's time before
     long long cache_words;     // per slot: language-cache words
     long long max_rows;        // per slot: rows of parents (and keys)
     int *order;                // the pending instances (null: 0 .. pending - 1)

@@ -188,8 +188,10 @@ def run_cfg4(count=4096, seed=0, tune_sample=1024, gen_workers=16, device=0) -> 
             "max_cost": max(costs) if costs else None,
             "time_to_minimal_ms": {"mean": float(np.mean([r.device_ms for r in res])),
                                    "max": float(np.max([r.device_ms for r in res])),
-                                   "note": "device time of each instance from its slot's set-up to its result"},
-            "launches": "one batch-start launch and one level-kernel launch for the whole batch",
+                                   "note": "device time on each instance: its pass over the small levels, and its slot's "
+                                           "from set-up to its result"},
+            "launches": "one small-level launch, one batch-start launch and one level-kernel launch for the "
+                        "whole batch",
             "autotune": {"best": best, "sample": tune_sample, "configs": len(table),
                          "worst_seconds": max(t["seconds"] for t in table)},
             "generation_s": t_gen}
