@@ -250,7 +250,8 @@ LTLG_API int ltlg_engine_level_starts(ltlg_engine *eng, int64_t *starts, int32_t
 LTLG_API int ltlg_engine_hold_slot(ltlg_engine *eng, const uint64_t *cs, int32_t n);
 
 /* Device building blocks, for kernel-level parity tests (device buffers are allocated
- * and freed inside; host arrays in and out). */
+ * and freed inside; host arrays in and out).  The operator is applied as each of the enumerator's
+ * paths does; bit 63 of an output word is set where two of them differ. */
 LTLG_API int ltlg_device_apply_op(int32_t op, const uint64_t *a, const uint64_t *b, const uint64_t *lenmask,
                                   int32_t n, int32_t count, uint64_t *out, uint64_t *out2, uint64_t *fp);
 

@@ -2,8 +2,9 @@
 // divide-and-conquer driver applies to every sub-formula (the reference's dc.py does it on
 // the host with bitarray, code/dc.py:136-187).  The string is parsed the way dc.py's bitVec
 // reads it (code/dc.py:136-183): "~(f)", "X(f)", "F(f)", "G(f)", "(f)&(g)", "(f)|(g)",
-// "(f)U(g)", single letters; the postfix program then runs on every trace in parallel with
-// the enumerator's own operators, reading the traces' step masks.
+// "(f)U(g)", single letters; the postfix program then runs on every trace in parallel on words in
+// natural order made from the step masks (unary_bits, until_bits; apply_op_kernel checks them against the
+// enumerator's operators on row words).
 #include <cuda_runtime.h>
 
 #include <cstring>

@@ -2254,7 +2254,32 @@ __global__ void walk_kernel(const u64 *parents, int nalpha, u64 found, const Ins
     out[1] = (u64)overflow;
 }
 
-// Operator + fingerprint on independent rows, for kernel-level parity tests.  One warp per row.
+// A candidate's word as each of the enumerator's paths makes it from row words (wop: an operator, or W_URL; unary
+// operators read r; m: length mask): the level kernel's units, its sweeps over wide rows, the small levels.  The
+// first one's, with bit 63 (0 in every CS) set where another differs.
+__device__ u64 word_of_every_path(int wop, u64 l, u64 r, u64 m) {
+    const bool un = wop == OP_NEG || wop == OP_X || wop == OP_F || wop == OP_G;
+    const u64 o = wop == OP_OR ? ~0ull : 0ull;
+    u64 unit = 0, sweep;
+    if (un) {
+        unit = row_unary(wop, r, m);
+        sweep = wop == OP_NEG ? sweep_word<SW_NEG>(l, r, m, o, false)
+                : wop == OP_X ? sweep_word<SW_X>(l, r, m, o, false)
+                : wop == OP_F ? sweep_word<SW_F>(l, r, m, o, false)
+                              : sweep_word<SW_G>(l, r, m, o, false);
+    } else {
+        const int t = wop == OP_AND ? 0 : wop == OP_OR ? 1 : wop == OP_U ? 2 : 3;
+        pair_words<M_ALL>(make_ulonglong2(l, 0), make_ulonglong2(r, 0), 0, 1u << t, [&](int, u64 w, u64) { unit = w; });
+        sweep = wop == OP_AND || wop == OP_OR ? sweep_word<SW_ANDOR>(l, r, m, o, false)
+                                              : sweep_word<SW_U>(l, r, m, o, wop == W_URL);
+    }
+    const u64 local = local_form(un, wop).word(l, r, m);
+    return unit | (unit != sweep || unit != local ? 1ull << 63 : 0ull);
+}
+// Operator + fingerprint on independent rows, for kernel-level parity tests: words come and go with position k in bit
+// k, and are row words in between.  Bit 63 of a result: the paths, or the two ways to make a length mask or (unary
+// operators and U in natural order, as formulas are evaluated on traces) to apply the operator, differ.  One warp per
+// row.
 __global__ void apply_op_kernel(int op, const u64 *a, const u64 *b, const u64 *wmeta, int n, int pitch, int count,
                                 u64 *out, u64 *out2, u64 *fp) {
     const int lane = threadIdx.x & 31;
@@ -2264,20 +2289,16 @@ __global__ void apply_op_kernel(int op, const u64 *a, const u64 *b, const u64 *w
     for (int i = lane; i < pitch; i += 32) {
         const u64 x = a[(u64)row * pitch + i], y = b ? b[(u64)row * pitch + i] : 0;
         const u64 m = wmeta[i];
-        u64 w = 0, w2 = 0;
-        switch (op) {
-        case OP_NEG:
-        case OP_X:
-        case OP_F:
-        case OP_G: w = unary_bits(op, x, m); break;
-        case OP_AND: w = x & y; break;
-        case OP_OR: w = x | y; break;
-        case OP_U:
-            w = until_bits(x, y);
-            w2 = until_bits(y, x);
-            break;
-        default: w = x; break;
-        }
+        const bool un = op == OP_NEG || op == OP_X || op == OP_F || op == OP_G;
+        const u64 xr = rev62(x), yr = rev62(y), mr = rev62(m);
+        u64 w = un ? word_of_every_path(op, 0ull, xr, mr) : word_of_every_path(op, xr, yr, mr);
+        u64 w2 = op == OP_U ? word_of_every_path(W_URL, xr, yr, mr) : 0ull;
+        bool differ = ((w | w2) >> 63) != 0ull || ((m & (m + 1ull)) == 0ull && row_lenmask(__popcll(m)) != mr);
+        w = rev62(w);
+        w2 = rev62(w2);
+        if (un) differ |= w != unary_bits(op, x, m);
+        if (op == OP_U) differ |= w != until_bits(x, y) || w2 != until_bits(y, x);
+        if (differ) w |= 1ull << 63;
         out[(u64)row * pitch + i] = w;
         if (out2) out2[(u64)row * pitch + i] = w2;
         const u64 key = (u64)(i + 1) * WEYL;

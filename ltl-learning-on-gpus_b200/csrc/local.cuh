@@ -221,17 +221,22 @@ struct LocalCand {
     }
     __device__ __forceinline__ u64 word(u64 x, u64 z, u64 m) const { return un ? row_unary(wop, z, m & LENMASK) : pair(x, z); }
 };
+__device__ __forceinline__ LocalCand local_form(bool un, int wop) {  // without its rows
+    LocalCand k;
+    k.l = k.r = nullptr;
+    k.wop = wop;
+    k.un = un;
+    k.rl = wop == W_URL;
+    k.n = wop == OP_AND ? 0ull : ~0ull;
+    k.u = wop == OP_U || wop == W_URL ? ~0ull : 0ull;
+    k.o = wop == OP_OR ? ~0ull : 0ull;
+    return k;
+}
 __device__ __forceinline__ LocalCand local_cand(const Local &S, const LocalUnit &x, int t) {
     const u64 pitch = (u64)S.A.pitch;
-    LocalCand k;
+    LocalCand k = local_form(x.g->mode == M_UNARY, local_wop(*x.g, t));
     k.l = reinterpret_cast<const ulonglong2 *>(S.A.cache + (u64)x.l * pitch);
     k.r = reinterpret_cast<const ulonglong2 *>(S.A.cache + (u64)x.r * pitch);
-    k.wop = local_wop(*x.g, t);
-    k.un = x.g->mode == M_UNARY;
-    k.rl = k.wop == W_URL;
-    k.n = k.wop == OP_AND ? 0ull : ~0ull;
-    k.u = k.wop == OP_U || k.wop == W_URL ? ~0ull : 0ull;
-    k.o = k.wop == OP_OR ? ~0ull : 0ull;
     return k;
 }
 // f(c, words of chunk c) over chunks c = gl, gl + P, ...  One chunk at a time: two or four in flight spill
