@@ -24,8 +24,8 @@
 // The find follows the reference's order: the reference runs a level's blocks one after the
 // other and stops after the first block that holds an accepting candidate
 // (code/ltli6463.cu:1232-1234), so here the find is the accepting candidate of the smallest
-// block position (an atomicMin on cost << 32 | position); items of later blocks are skipped once
-// a find is known, items of earlier blocks still run.
+// block position (an atomicMin on cost << 32 | position); once a find is known, items of later blocks
+// are skipped and fused items run without the operators of later blocks; earlier blocks still run.
 //
 // Semantics follow MojtabaValizadeh/ltl-learning-on-gpus, code/ltli6463.cu:
 //   acceptance ......... :240-243 (positives need bit 0 set, negatives clear)
@@ -75,8 +75,8 @@ struct Slot {
     int split;                // units per row (left groups of the tile; a small level's unary operators)
     int lefts;                // binary: left rows of a unit
     int units;                // nrows * split: what the consumers take
-    int overflowed;           // the cache had overflowed when the item was claimed (or a claim here
-                              // overflowed): the rows' new CSs take no hash slots
+    int overflowed;           // the cache had overflowed when the item was claimed: the rows' new CSs take no
+                              // hash slots
     InstArgs args;            // its arguments as they were when the item was claimed (a batch slot's
                               // arguments change when it takes the next instance)
 };
@@ -426,8 +426,8 @@ __device__ void take_over(const InstArgs &A, InstCtl *C, const Gen &g, int t, u6
 // published before any lane waits on another warp's publication, so waits cannot cycle.
 template <int NC, bool WIDE, class Gen>
 __device__ __forceinline__ void resolve(const InstArgs &A, InstCtl *C, int cost, const Gen &g, u64 fp, bool active,
-                                        u64 parent, u64 kh, u64 kl, u64 prio, u32 anyp, u32 anyn, int *overflowed,
-                                        u32 ring, int lane) {
+                                        u64 parent, u64 kh, u64 kl, u64 prio, u32 anyp, u32 anyn, u32 ring,
+                                        int lane) {
     int state = active ? S_PROBE : S_DONE;
     const u64 tagbits = (fp >> 40) << 40;
     const u64 genbits = (u64)A.gen << 32;
@@ -667,7 +667,8 @@ __device__ __forceinline__ bool known_duplicate(const InstArgs &A, int wop, u32 
 
 // Fingerprints, acceptance, the find record, uniqueness for NC candidates of one warp.
 // fails[t]: this lane's words of candidate t at position 0 (fails2); bp, bn: the row statistics'
-// bits (pmiss2, nhit2), kept only when the learn counts them.  pos_of(t): block position of candidate t (the find record is per block).
+// bits (pmiss2, nhit2), kept only when the learn counts them.  pos_of(t): block position of candidate t
+// (the find record is per block).
 template <int NC, bool WIDE, class Gen, class ParentOf, class PosOf, class TidOf>
 __device__ __forceinline__ void finish(const InstArgs &A, InstCtl *C, Slot &sl, const Gen &g, u64 (&h)[NC],
                                        u32 (&fails)[NC], u32 bp, u32 bn, u32 valid, ParentOf parent_of, PosOf pos_of,
@@ -729,15 +730,14 @@ __device__ __forceinline__ void finish(const InstArgs &A, InstCtl *C, Slot &sl, 
         const bool same_level = !un && sl.e_l0 == sl.e_r0;
         mine = !known_duplicate(A, op, x, un ? x : y, px, py, same_level);
     }
-    resolve<NC, WIDE>(A, C, cost, g, fp, mine, myparent, kh, kl, prio, anyp, anyn,
-                      &sl.overflowed, ring, lane);
+    resolve<NC, WIDE>(A, C, cost, g, fp, mine, myparent, kh, kl, prio, anyp, anyn, ring, lane);
 }
 
 // ---------------------------------------------------------------- rows
 // Binary unit: right row r (at R) against nl left rows of the slot's tile (row l_first and up),
 // every operator of MODE on each pair: NL * mode_ops(MODE) candidates.  Chunks are 16 bytes (two
-// words); two are in flight per lane, or four on wide rows (stream).  Positives are the first npos words, so acceptance needs no
-// metadata.
+// words); two are in flight per lane, or four on wide rows (stream).  Positives are the first npos words,
+// so acceptance needs no metadata.
 //
 // The sweep is bound by integer issue (ALU and the wide multiply-add), so it is laid out to share
 // work: one load of the pair's chunks feeds every operator (& | l U r r U l share l | r), the

@@ -241,65 +241,39 @@ __device__ __forceinline__ LocalCand local_cand(const Local &S, const LocalUnit 
 }
 // f(c, words of chunk c) over chunks c = gl, gl + P, ...  One chunk at a time: two or four in flight spill
 // (64 registers) and made a level of 732 candidates take 34 instead of 24 us.
-constexpr int LCH = 1;
 template <class F>
 __device__ __forceinline__ void local_words(const Local &S, const LocalCand &k, int gl, int P, int nch, F f) {
 #pragma unroll 1
-    for (int c0 = gl; c0 < nch; c0 += LCH * P) {
-        ulonglong2 l[LCH], r[LCH];
-#pragma unroll
-        for (int u = 0; u < LCH; ++u) {
-            const int c = c0 + u * P;
-            if (c < nch) {
-                r[u] = k.r[c];
-                l[u] = k.un ? r[u] : k.l[c];
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < LCH; ++u) {
-            const int c = c0 + u * P;
-            if (c >= nch) break;
-            f(c, k.word(l[u].x, r[u].x, S.meta[2 * c]), k.word(l[u].y, r[u].y, S.meta[2 * c + 1]));
-        }
+    for (int c = gl; c < nch; c += P) {
+        const ulonglong2 r = k.r[c], l = k.un ? r : k.l[c];
+        f(c, k.word(l.x, r.x, S.meta[2 * c]), k.word(l.y, r.y, S.meta[2 * c + 1]));
     }
 }
 
 // Sums and acceptance of one unit over this lane's chunks (first lane gl of P lanes).
 template <int MODE, int HK>
 __device__ __forceinline__ void local_eval(const Local &S, const LocalUnit &x, int gl, int P, u64 (&h)[4], u32 (&fails)[4]) {
-    constexpr int CH = 1;  // chunks in flight
     const int nch = S.A.pitch >> 1, npos = S.A.npos, n = S.A.n, opmask = x.g->op;
     const u64 pitch = (u64)S.A.pitch;
     const ulonglong2 *R = reinterpret_cast<const ulonglong2 *>(S.A.cache + (u64)x.r * pitch);
     const ulonglong2 *L = reinterpret_cast<const ulonglong2 *>(S.A.cache + (u64)x.l * pitch);
 #pragma unroll 1
-    for (int c0 = gl; c0 < nch; c0 += CH * P) {
-        ulonglong2 rv[CH], lv[CH];
+    for (int c = gl; c < nch; c += P) {
+        const ulonglong2 rv = R[c];
+        const u64 k = (2ull * (u64)c + 1ull) * WEYL;
+        const u32 p0 = 2 * c < npos ? ROW_BIT0_HI : 0u, p1 = 2 * c + 1 < npos ? ROW_BIT0_HI : 0u;
+        const bool v0 = 2 * c < n, v1 = 2 * c + 1 < n;
+        auto take = [&](int t, u64 w0, u64 w1) {
+            h[t] += hw<HK>(w0, k, v0) + hw<HK>(w1, k + WEYL, v1);
+            fails[t] |= fails2(w0, w1, p0, p1);
+        };
+        if constexpr (MODE == M_UNARY) {
+            const u64 m0 = S.meta[2 * c] & LENMASK, m1 = S.meta[2 * c + 1] & LENMASK;
 #pragma unroll
-        for (int u = 0; u < CH; ++u)
-            if (c0 + u * P < nch) {
-                rv[u] = R[c0 + u * P];
-                if (MODE != M_UNARY) lv[u] = L[c0 + u * P];
-            }
-#pragma unroll
-        for (int u = 0; u < CH; ++u) {
-            const int c = c0 + u * P;
-            if (c >= nch) break;
-            const u64 k = (2ull * (u64)c + 1ull) * WEYL;
-            const u32 p0 = 2 * c < npos ? ROW_BIT0_HI : 0u, p1 = 2 * c + 1 < npos ? ROW_BIT0_HI : 0u;
-            const bool v0 = 2 * c < n, v1 = 2 * c + 1 < n;
-            auto take = [&](int t, u64 w0, u64 w1) {
-                h[t] += hw<HK>(w0, k, v0) + hw<HK>(w1, k + WEYL, v1);
-                fails[t] |= fails2(w0, w1, p0, p1);
-            };
-            if constexpr (MODE == M_UNARY) {
-                const u64 m0 = S.meta[2 * c] & LENMASK, m1 = S.meta[2 * c + 1] & LENMASK;
-#pragma unroll
-                for (int t = 0; t < 4; ++t)
-                    if ((opmask >> t) & 1) take(t, row_unary(unary_slot_op(t), rv[u].x, m0), row_unary(unary_slot_op(t), rv[u].y, m1));
-            } else {
-                pair_words<MODE>(lv[u], rv[u], 0, 15u, take);
-            }
+            for (int t = 0; t < 4; ++t)
+                if ((opmask >> t) & 1) take(t, row_unary(unary_slot_op(t), rv.x, m0), row_unary(unary_slot_op(t), rv.y, m1));
+        } else {
+            pair_words<MODE>(L[c], rv, 0, 15u, take);
         }
     }
 }
