@@ -69,7 +69,7 @@ struct Slot {
     int upos[4];              // unary: block position of each slot operator; fused binary: of & | U
     int cost;
     int check_only;
-    int live;                 // operators of the entry still to run (live_ops); 0: remaining rows are skipped
+    int found;                // first block with a find in the level: what comes behind it is left out (live_ops)
     int inst;                 // the item's instance (index into Launch::args)
     int trace_first;          // the producer's first item of this plan (level stamps)
     int split;                // units per row (left groups of the tile; a small level's unary operators)
@@ -81,15 +81,15 @@ struct Slot {
                               // arguments change when it takes the next instance)
 };
 
-// How many of an entry's operators are still worth running once the level has a find in block `found`: those whose
-// block comes before it (find_first: none), which are the first ones, as a fused entry's blocks & | U come in this
-// order.  Other entries go on as a whole or not at all (a fused unary entry until its first block is passed).
-__host__ __device__ __forceinline__ int entry_ops(int kind) { return kind == ENT_ALL ? 3 : kind == ENT_AO ? 2 : 1; }
-__device__ __forceinline__ int live_ops(int kind, int pos, const int (&upos)[4], int found, bool find_first) {
-    if (find_first || pos >= found) return 0;
-    int n = 1;
-    while (n < entry_ops(kind) && upos[n] < found) ++n;
-    return n;
+// The first operators of an entry (fused ones run & | U, whose blocks come in this order) that are still worth running
+// once the level has a find in block `found` (NO_BLOCK: none; -1: any find ends it): those whose block comes before
+// it.  Bookkeeping per unit kept to one load beside the unit's number: learns of 60 to 600 us took 1.2% longer on
+// average when each unit had its own count of operators, 0.5% so.
+// Other entries go on as a whole or not at all (a fused unary entry until its first block is passed).
+constexpr int NO_BLOCK = POS_NONE;
+__device__ __forceinline__ int live_ops(int kind, int pos, const int *upos, int found) {
+    if (pos >= found) return 0;
+    return kind == ENT_ALL ? 1 + (upos[1] < found) + (upos[2] < found) : kind == ENT_AO ? 1 + (upos[1] < found) : 1;
 }
 
 // ---------------------------------------------------------------- candidate generators
@@ -695,7 +695,7 @@ __device__ __forceinline__ void finish(const InstArgs &A, InstCtl *C, Slot &sl, 
             }
             // the item's remaining rows are skipped, or run under fewer operators, only when the search ends
             // at this level
-            if (A.stop_at_found) atomicMin(&sl.live, live_ops(sl.kind, sl.pos, sl.upos, p, A.find_first != 0));
+            if (A.stop_at_found) atomicMin(&sl.found, A.find_first ? -1 : p);
         }
         __syncwarp();
         if (A.stop_at_found) return;  // this level is the last one; its candidates need no dedupe
@@ -1658,15 +1658,17 @@ __device__ __noinline__ void next_instance(BatchDev &B, int s, bool finishing, i
 __device__ __forceinline__ Slot *slot_at(unsigned char *smem, int s) { return reinterpret_cast<Slot *>(smem) + s; }
 
 // Item `item` of entry e (cached in shared memory) into slot sl.  Returns the tile bytes to copy
-// (0 for a unary item or a skipped one).  `live` of the entry's operators are run.
+// (0 for a unary item or a skipped one).
 __device__ __forceinline__ u32 fill_slot(Slot &sl, int inst, const Entry &e, long long item, int tile, int rc,
-                                         int ur, int cost, int check_only, long long plan_items, int live,
+                                         int ur, int cost, int check_only, long long plan_items, int found,
                                          int pitch) {
     const long long local = item - e.item0;
+    const int live = live_ops(e.kind, e.pos, e.upos, found);
     const bool skip = live == 0;
     sl.inst = inst;
     // a fused entry of which only & | or & are left is the smaller entry of these
-    sl.kind = skip || live == entry_ops(e.kind) ? e.kind : live == 2 ? (int)ENT_AO : (int)ENT_ONE;
+    const bool fused = e.kind == ENT_ALL || e.kind == ENT_AO;
+    sl.kind = skip || !fused ? e.kind : live == 3 ? (int)ENT_ALL : live == 2 ? (int)ENT_AO : (int)ENT_ONE;
     sl.pos = e.pos;
     for (int j = 0; j < 4; ++j) sl.upos[j] = e.upos[j];
     sl.cost = cost;
@@ -1675,7 +1677,7 @@ __device__ __forceinline__ u32 fill_slot(Slot &sl, int inst, const Entry &e, lon
     sl.next_row = 0;
     sl.rows_done = 0;
     sl.evals = 0;
-    sl.live = live;
+    sl.found = found;
     sl.e_l0 = e.l0;
     sl.e_r0 = e.r0;
     sl.e_R = e.r1 - e.r0;
@@ -1895,16 +1897,13 @@ __device__ void producer(const Launch &L, unsigned char *smem, u64 *tiles, int l
         }
         // skip rule: operators whose block comes after a find of this level (or any find, find_first)
         const bool found_here = pc.a.stop_at_found && fk != NO_FIND && (int)(fk >> 32) == pc.cost;
-        const int live = found_here ? live_ops(pc.e.kind, pc.e.pos, pc.e.upos, (int)(u32)fk, pc.a.find_first != 0)
-                                    : entry_ops(pc.e.kind);
-        const bool skip = live == 0;
+        const int found = !found_here ? NO_BLOCK : pc.a.find_first ? -1 : (int)(u32)fk;
+        const bool skip = pc.e.pos >= found;
         // the same rule for the remaining rows of the items of this level still in this CTA's slots (the slot
         // the producer is about to fill is not in flight)
         if (found_here && lane < S && lane != s) {
             Slot &o = *slot_at(smem, lane);
-            const int kind = *(volatile int *)&o.kind;
-            if (kind != 0 && o.inst == inst && o.cost == pc.cost)
-                atomicMin(&o.live, live_ops(kind, o.pos, o.upos, (int)(u32)fk, pc.a.find_first != 0));
+            if (*(volatile int *)&o.kind != 0 && o.inst == inst && o.cost == pc.cost) atomicMin(&o.found, found);
         }
         {
             constexpr int AW = sizeof(InstArgs) / 8;
@@ -1914,7 +1913,7 @@ __device__ void producer(const Launch &L, unsigned char *smem, u64 *tiles, int l
         }
         if (lane == 0) {
             const u32 bytes = fill_slot(sl, inst, pc.e, item, L.tile, pc.rc, pc.ur, pc.cost, pc.check_only,
-                                        pc.plan_items, live, pc.a.pitch);
+                                        pc.plan_items, found, pc.a.pitch);
             sl.trace_first = pc.trace_first;
             sl.overflowed = ovf ? 1 : 0;
             // units: a right row with unit_lefts of the tile's left rows; at a small level one left
@@ -1979,12 +1978,17 @@ __device__ __forceinline__ int take_rows(Slot &sl, int kind, const ulonglong2 *t
     int out = SLOT_NEXT;
     for (;;) {
         unsigned idx = 0;
-        if (lane == 0) idx = atomicAdd(&sl.next_row, 1u);
+        int live = 3;
+        if (lane == 0) {
+            idx = atomicAdd(&sl.next_row, 1u);
+            const int found = *(volatile int *)&sl.found;
+            if (found != NO_BLOCK) live = live_ops(kind, sl.pos, sl.upos, found);
+        }
         idx = __shfl_sync(FULL, idx, 0);
+        live = __shfl_sync(FULL, live, 0);
         if ((int)idx >= sl.units) break;
         if (idx == 0 && sl.trace_first && lane == 0)
             atomicCAS(A.level_ns + (u64)sl.cost * LEVEL_TRACE + LT_STARTED, 0ull, globaltimer());
-        const int live = __shfl_sync(FULL, *(volatile int *)&sl.live, 0);
         if (live) {
             const int split = sl.split, part = (int)idx % split;
             const long long r = sl.row0 + (int)idx / split;
@@ -2000,7 +2004,7 @@ __device__ __forceinline__ int take_rows(Slot &sl, int kind, const ulonglong2 *t
                 const long long lf = sl.l_first + first;
                 if (kind == ENT_ALL && live == 3)
                     binary_unit<M_ALL, unit_lefts<TL>(M_ALL), HK, WIDE>(A, C, sl, t0, nl, lf, rp, r, ring, lane);
-                else if ((kind == ENT_ALL || kind == ENT_AO) && live == 2)
+                else if ((kind == ENT_ALL || kind == ENT_AO) && live >= 2)
                     binary_unit<M_AO, unit_lefts<TL>(M_AO), HK, WIDE>(A, C, sl, t0, nl, lf, rp, r, ring, lane);
                 else if (kind == ENT_U)
                     binary_unit<M_U, unit_lefts<TL>(M_U), HK, WIDE>(A, C, sl, t0, nl, lf, rp, r, ring, lane);

@@ -45,7 +45,8 @@ struct Local {
     unsigned char fail[LC];    // F_* bits, then 1: differs from its match
     unsigned short claim[LC], verify[LC], retry[2][LC];
     unsigned short ul[LC / 4], ur[LC / 4];  // the round's units: operand rows,
-    unsigned char useg[LC / 4];             // segment
+    unsigned char useg[LC / 4];             // segment,
+    unsigned char uops[LC / 4];             // candidates (operators) to evaluate
     u32 nclaim, nverify, nretry[2];
     LocalSeg seg[LSEGS];
     int ls[LCOST + 3];
@@ -195,6 +196,14 @@ __device__ __forceinline__ void local_decode(Local &S, int u, int unit) {
     S.ul[u] = (unsigned short)(g.l0 + (int)l);
     S.ur[u] = (unsigned short)(g.r0 + (int)(q - l * (u32)g.nr));
     S.useg[u] = (unsigned char)lo;
+    // once a round has found and the search ends here, only the operators whose blocks come before the find
+    u32 ops = (u32)g.op;
+    if (S.A.stop_at_found && S.found_key != ~0ull) {
+        for (int t = 0; t < 4; ++t)
+            if (g.upos[t] >= (int)(S.found_key >> 32)) ops &= ~(1u << t);
+        if (ops != (u32)g.op) atomicAdd(&S.skipped, (u32)__popc((u32)g.op & ~ops));
+    }
+    S.uops[u] = (unsigned char)ops;
 }
 __device__ __forceinline__ LocalUnit local_unit(const Local &S, int u) {
     return LocalUnit{&S.seg[S.useg[u]], (int)S.ul[u], (int)S.ur[u]};
@@ -334,10 +343,6 @@ __device__ void local_level(Local &S, int c, int tid) {
     const int gl = lane & (P - 1), per_warp = 32 / P, group = tid / P, ngroups = LT / P;
     for (int u0 = 0; u0 < S.units; u0 += LC / 4) {
         const int nu = min(LC / 4, S.units - u0);
-        // Once a round has found and the search ends here, the later ones run the operators whose blocks come
-        // before the find, for acceptance only: nothing of the level is an operand any more.
-        const bool over = A.stop_at_found && S.found_key != ~0ull;
-        const int found = (int)(S.found_key >> 32);
         if (tid < nu) local_decode(S, tid, u0 + tid);
         __syncthreads();
         // fingerprints and acceptance
@@ -345,18 +350,12 @@ __device__ void local_level(Local &S, int c, int tid) {
             const int u = b + lane / P;
             u64 h[4] = {0, 0, 0, 0};
             u32 fails[4] = {0, 0, 0, 0}, valid = 0;
-            if (u < nu) {
+            if (u < nu && S.uops[u]) {
                 const LocalUnit x = local_unit(S, u);
-                valid = (u32)x.g->op;
-                if (over) {
-#pragma unroll
-                    for (int t = 0; t < 4; ++t)
-                        if (x.g->upos[t] >= found) valid &= ~(1u << t);
-                    if (gl == 0) atomicAdd(&S.skipped, (u32)__popc((u32)x.g->op & ~valid));
-                }
-                if (valid && x.g->mode == M_UNARY)
+                valid = S.uops[u];
+                if (x.g->mode == M_UNARY)
                     local_eval<M_UNARY, HK>(S, x, gl, P, h, fails);
-                else if (valid)
+                else
                     local_eval<M_ALL, HK>(S, x, gl, P, h, fails);
             }
             __syncwarp();
@@ -393,7 +392,6 @@ __device__ void local_level(Local &S, int c, int tid) {
                 atomicMin(&S.found_key, mine[q]);
                 if (A.stop_at_found) continue;  // the last level: no dedupe
             }
-            if (over) continue;
             local_probe(S, j, (u32)S.sum[j] & (LTAB - 1));
         }
         __syncthreads();
