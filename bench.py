@@ -435,8 +435,9 @@ def run_ours(a):
                        "e2e": "unique CS / CUDA-event time of ltlg_batch_learn on host traces"},
             "time_to_minimal_formula_ms": {"mean": statistics.mean(ttm), "median": statistics.median(ttm),
                                            "max": max(ttm), "min_cost": min(costs), "max_cost": max(costs),
-                                           "note": "device time of each instance inside the batch launch, "
-                                                   "from its slot's set-up to its result"},
+                                           "note": "device time on each instance inside the batch call: its pass over "
+                                                   "the small levels where it has one, and its slot's from set-up to "
+                                                   "its result"},
             "candidate_cs_per_s": tot[3] / kern_t,
             "e2e": {"value": tot[0] / step_t, "unit": UNIT, "h2d_bytes_per_step": h2d // K,
                     "d2h_bytes_per_step": d2h // K, "candidate_cs_per_s": tot[1] / step_t,
